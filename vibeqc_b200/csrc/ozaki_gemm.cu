@@ -25,8 +25,9 @@
 //   K-block: warp 6 loads the ns B-slice tiles as one group (two groups in
 //   flight), warp 0 loads the ns A-slice tiles one by one (six in flight) in
 //   the interleaved order 0, ns-1, 1, ns-2, ... so that heavy (many pairs) and
-//   light slices alternate; warp 1 issues the MMAs (A slice s with the B
-//   slices t, s + t <= ns + 1, into accumulator g = s + t); warps 2-5 drain
+//   light slices alternate; warps 1 and 7 issue the MMAs (A slice s with the B
+//   slices t, s + t <= ns + 1, into accumulator g = s + t; the slices of an
+//   issuer's accumulators stacked into one MMA); warps 2-5 drain
 //   the accumulators (TMEM -> int32 -> FP64), scale, stage the tile in the
 //   idle A ring and store whole rows.
 //   With `upper`, B[n][k] = 0 for k > n and a column tile reads only the
@@ -52,9 +53,11 @@ constexpr int kWRing = 2;
 constexpr int A_TILE = BM * BKB;              // 16 KB
 constexpr int B_TILE = BN * BKB;              // 8 KB
 constexpr int B_GROUP = kMaxSlices * B_TILE;  // 56 KB
-// MMA issuers: the int8 MMA costs ~150 cycles of issue per instruction whatever its N, so
-// two issuing warps (accumulators split by parity) keep more of them in flight
+// MMA issuers: issuer 0 owns the accumulators g < kGroup0, issuer 1 the others (an accumulator's
+// MMAs must come from one thread to stay ordered).  A stacked MMA spans at most N = 256 columns,
+// four accumulators; at 7 slices the issuers send 4 and 7 MMAs per K-step for the 28 slice pairs
 constexpr int kIssuers = 2;
+constexpr int kGroup0 = 4;
 constexpr int kThreads = 32 * (7 + kIssuers - 1);  // A producer, issuer 0, 4 epilogue, B producer, issuer 1
 constexpr int kTmemCols = 512;                // ns (<= 7) accumulators of BN columns
 
@@ -170,9 +173,8 @@ __device__ __forceinline__ void tmem_ld16_i32(uint32_t taddr, int (&v)[16]) {
 // j-th A slice of a K-block in issue order: 0, ns-1, 1, ns-2, ...
 __device__ __forceinline__ int slice_order(int j, int ns) { return (j & 1) ? ns - 1 - (j >> 1) : (j >> 1); }
 
-// D = S32 (bits 4-5 = 2), A = B = signed 8-bit (1), both K-major, N >> 3, M >> 4
-constexpr uint32_t kIdescI8 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-                              ((uint32_t)(BM >> 4) << 24);
+// D = S32 (bits 4-5 = 2), A = B = signed 8-bit (1), both K-major, M >> 4; N >> 3 is added per MMA
+constexpr uint32_t kIdescI8 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BM >> 4) << 24);
 
 
 // Persistent over output tiles: each CTA (one per SM: 512 TMEM columns)
@@ -274,7 +276,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
   } else if (warp == 1 || warp >= 7) {
-    const int me = warp == 1 ? 0 : warp - 6;  // issuer index: accumulators g with g % kIssuers == me
+    const int me = warp == 1 ? 0 : warp - 6;  // issuer index
+    const int gbeg = me == 0 ? 0 : kGroup0, gend = me == 0 ? min(ns, kGroup0) : ns;
     if (lane == 0) {  // MMA issuer
       int ai = 0, gkb = 0, it = 0;
       bool ok = true;
@@ -312,17 +315,23 @@ __global__ void __launch_bounds__(kThreads, 1)
             // slices are 0-based here: pair (s, t) with s + t <= ns - 1 feeds
             // accumulator g = s + t (weight 2^-7(g+2)); slice 0 comes first in
             // the issue order, so its first K-step initialises every accumulator
+            // The B slices lie one after another and so do the accumulators
+            // they feed (g = s + t), so the slices t with g in this issuer's
+            // range [g0, g1) are ONE MMA with N = 64 (g1 - g0): the A tile is
+            // read from shared memory once per MMA instead of once per pair
+            // (an N = 64 MMA reads 6 KB for 32 cycles of math, 48 at 128 B a
+            // cycle).  8 x (H2O)10: 7.67 -> 5.04 ms.
             const uint64_t adesc0 = smem_desc(smem_u32(abuf + as * A_TILE));
-            const uint32_t first = (kb == 0 && s == 0) ? 0u : 1u;
-            uint32_t dt = tmem + (uint32_t)(s * BN);
-            uint64_t bdesc = bdesc0;
-            for (int tt = 0; tt + s < ns; ++tt, dt += BN, bdesc += B_TILE >> 4) {
-              if ((s + tt) % kIssuers != me) continue;
-              if (first) mma_i8_acc(dt, adesc0, bdesc, kIdescI8);
-              else mma_i8(dt, adesc0, bdesc, kIdescI8, 0u);
-              mma_i8_acc(dt, adesc0 + 2, bdesc + 2, kIdescI8);
-              mma_i8_acc(dt, adesc0 + 4, bdesc + 4, kIdescI8);
-              mma_i8_acc(dt, adesc0 + 6, bdesc + 6, kIdescI8);
+            const int g0 = max(s, gbeg);
+            if (g0 < gend) {
+              const uint32_t dt = tmem + (uint32_t)(g0 * BN);
+              const uint64_t bdesc = bdesc0 + (uint64_t)(g0 - s) * (B_TILE >> 4);
+              const uint32_t idesc = kIdescI8 | ((uint32_t)((gend - g0) * BN >> 3) << 17);
+              if (kb != 0 || s != 0) mma_i8_acc(dt, adesc0, bdesc, idesc);
+              else mma_i8(dt, adesc0, bdesc, idesc, 0u);
+              mma_i8_acc(dt, adesc0 + 2, bdesc + 2, idesc);
+              mma_i8_acc(dt, adesc0 + 4, bdesc + 4, idesc);
+              mma_i8_acc(dt, adesc0 + 6, bdesc + 6, idesc);
             }
             mma_commit(ae0 + 8 * as);
           }
@@ -437,11 +446,56 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
+// Digits of one scaled element y (|y| < 1 up to the clamp): repeated
+// round-to-nearest of 128 y, clamped to +-127, remainder carried on.
+__device__ __forceinline__ void slice_digits_clamped(double y, int ns, int (&dig)[kMaxSlices]) {
+#pragma unroll
+  for (int s = 0; s < kMaxSlices; ++s) {
+    if (s < ns) {
+      y *= 128.0;
+      const double a = fmin(127.0, fmax(-127.0, rint(y)));
+      y -= a;
+      dig[s] = (int)a;
+    }
+  }
+}
+
+// The same digits without the clamp, three FP64 operations each: adding
+// 1.5 * 2^52 rounds 128 y to the nearest integer (ties to even, as rint) and
+// leaves it in the low word of the sum.  Only an element whose digit reaches
+// +-128 (|y| within 2^-8 of 1, at most a few per row) needs the clamped form.
+template <int NS>
+__device__ __forceinline__ void slice_digits(double y0, int ns, int (&dig)[kMaxSlices]) {
+  constexpr double kMagic = 6755399441055744.0;
+  double y = y0;
+  bool over = false;
+#pragma unroll
+  for (int s = 0; s < kMaxSlices; ++s) {
+    if (s < (NS ? NS : ns)) {
+      const double t = fma(y, 128.0, kMagic);
+      y = fma(y, 128.0, kMagic - t);
+      dig[s] = __double2loint(t);
+      over |= dig[s] > 127 || dig[s] < -127;
+    }
+  }
+  if (over) slice_digits_clamped(y0, ns, dig);
+}
+
 // rows of src (FP64, optionally times a per-column power-of-two scale) ->
-// ns int8 slices and the row exponent; one warp per row
-__global__ void slice_rows_kernel(const double* __restrict__ src, int nmol, long long rows, int cols,
-                                  long long ld, long long mol_stride, const double* __restrict__ col_scale,
-                                  int ns, int8_t* __restrict__ dst, int ldd, int* __restrict__ exps) {
+// ns int8 slices and the row exponent; one warp per row.  Bound by the 8 B
+// read and ns B written per element.  A lane takes four consecutive columns
+// (two 16-byte loads, one 4-byte store per slice: whole 128-byte lines per
+// warp; one-byte stores and the rounding / clamping / conversion chain held
+// the earlier form to 1.5 TB/s).  The row maximum enters only through its
+// exponent, so the first pass is an integer maximum over exponent fields.
+// 8 x (H2O)10: 2.65 -> 1.39 ms, 2.9 TB/s; the 21 FP64 operations an element
+// takes are next.
+// VEC: 16-byte aligned source and scale rows and 4-byte aligned slice rows.
+template <bool VEC, int NS>
+__global__ void __launch_bounds__(256)
+    slice_rows_kernel(const double* __restrict__ src, int nmol, long long rows, int cols, long long ld,
+                      long long mol_stride, const double* __restrict__ col_scale, int ns,
+                      int8_t* __restrict__ dst, int ldd, int* __restrict__ exps) {
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
   const int lane = threadIdx.x & 31;
   for (long long gr = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -449,22 +503,65 @@ __global__ void slice_rows_kernel(const double* __restrict__ src, int nmol, long
     const long long z = gr / rows, r = gr - z * rows;
     const double* x = src + z * mol_stride + r * ld;
     const double* sc = col_scale ? col_scale + z * cols : nullptr;
-    double mx = 0.0;
-    for (int c = lane; c < cols; c += 32) mx = fmax(mx, fabs(sc ? x[c] * sc[c] : x[c]));
+    // four scaled columns c .. c + 3 (zero past the end)
+    auto load4 = [&](int c, double (&v)[4]) {
+      if (VEC && c + 4 <= cols) {
+        const double2 p = *reinterpret_cast<const double2*>(x + c);
+        const double2 q = *reinterpret_cast<const double2*>(x + c + 2);
+        v[0] = p.x, v[1] = p.y, v[2] = q.x, v[3] = q.y;
+        if (sc) {
+          const double2 a = __ldg(reinterpret_cast<const double2*>(sc + c));
+          const double2 b = __ldg(reinterpret_cast<const double2*>(sc + c + 2));
+          v[0] *= a.x, v[1] *= a.y, v[2] *= b.x, v[3] *= b.y;
+        }
+      } else {
 #pragma unroll
-    for (int o = 16; o; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    int e = 0;
-    if (mx > 0.0) frexp(mx, &e);  // mx < 2^e
+        for (int e = 0; e < 4; ++e) v[e] = c + e < cols ? (sc ? x[c + e] * __ldg(sc + c + e) : x[c + e]) : 0.0;
+      }
+    };
+    int field = 0;
+#pragma unroll 4
+    for (int c = 4 * lane; c < cols; c += 128) {
+      double v[4];
+      load4(c, v);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) field = max(field, __double2hiint(v[e]) & 0x7ff00000);
+    }
+    field = __reduce_max_sync(0xffffffffu, field);
+    int e = (field >> 20) - 1022;  // max |row| < 2^e for a normal maximum (frexp's exponent)
+    const bool odd = field == 0 || field == 0x7ff00000;  // zero, subnormal or non-finite maximum
+    if (odd) {
+      double mx = 0.0;
+      for (int c = lane; c < cols; c += 32) mx = fmax(mx, fabs(sc ? x[c] * sc[c] : x[c]));
+#pragma unroll
+      for (int o = 16; o; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      e = 0;
+      if (mx > 0.0) frexp(mx, &e);
+    }
     const double inv = ldexp(1.0, -e);
     int8_t* d = dst + (z * ns * rows + r) * (long long)ldd;
     const long long sstride = rows * (long long)ldd;
-    for (int c = lane; c < cols; c += 32) {
-      double y = (sc ? x[c] * sc[c] : x[c]) * inv;
-      for (int s = 0; s < ns; ++s) {
-        y *= 128.0;
-        const double a = fmin(127.0, fmax(-127.0, rint(y)));
-        y -= a;
-        d[s * sstride + c] = (int8_t)(int)a;
+    for (int c = 4 * lane; c < cols; c += 128) {
+      double v[4];
+      load4(c, v);
+      int dig[4][kMaxSlices];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (odd) slice_digits_clamped(v[k] * inv, ns, dig[k]);
+        else slice_digits<NS>(v[k] * inv, ns, dig[k]);
+      }
+      if (VEC && c + 4 <= cols) {
+#pragma unroll
+        for (int s = 0; s < kMaxSlices; ++s)
+          if (s < (NS ? NS : ns))
+            *reinterpret_cast<char4*>(d + s * sstride + c) =
+                make_char4((char)dig[0][s], (char)dig[1][s], (char)dig[2][s], (char)dig[3][s]);
+      } else {
+#pragma unroll
+        for (int s = 0; s < kMaxSlices; ++s)
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (s < (NS ? NS : ns) && c + k < cols) d[s * sstride + c + k] = (int8_t)dig[k][s];
       }
     }
     if (lane == 0) exps[z * rows + r] = e;
@@ -503,8 +600,14 @@ extern "C" int vqc_ozaki_slice_rows(const double* src, int32_t nmol, int64_t row
     return fail(VQC_STATUS_INVALID_ARGUMENT, "ozaki_slice_rows: bad argument");
   const long long total = (long long)nmol * rows;
   const long long blocks = std::min<long long>((total + 7) / 8, 148LL * 64);
-  oz::slice_rows_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
-      src, nmol, rows, cols, ld, mol_stride, col_scale, nslices, dst, ldd, exps);
+  const bool vec = reinterpret_cast<uintptr_t>(src) % 16 == 0 && ld % 2 == 0 && mol_stride % 2 == 0 &&
+                   reinterpret_cast<uintptr_t>(dst) % 4 == 0 && ldd % 4 == 0 &&
+                   (!col_scale || (reinterpret_cast<uintptr_t>(col_scale) % 16 == 0 && cols % 2 == 0));
+  auto kern = nslices == oz::kMaxSlices
+                  ? (vec ? oz::slice_rows_kernel<true, oz::kMaxSlices> : oz::slice_rows_kernel<false, oz::kMaxSlices>)
+                  : (vec ? oz::slice_rows_kernel<true, 0> : oz::slice_rows_kernel<false, 0>);
+  kern<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(src, nmol, rows, cols, ld, mol_stride,
+                                                           col_scale, nslices, dst, ldd, exps);
   count_launch();
   return cuda_status(cudaGetLastError(), "ozaki_slice_rows");
 }
