@@ -228,6 +228,22 @@ int vqc_sp2_update(const double* x, const double* x2, double* xout, int32_t nmol
                    double nocc, double tol, int32_t* done, void* stream);
 
 /*
+ * Whole SP2 purification of nmol symmetric n*n blocks fo (row-major,
+ * contiguous; the mean of fo and its transpose is used) in one launch:
+ * Gershgorin map to [0, 1], then X^2 or 2X - X^2 steps as above until
+ * |tr X - tr X^2| < tol or max_steps steps; out receives X, the projector onto
+ * the lowest nocc eigenvectors.  path: 0 picks by size; 1 one CTA per molecule
+ * (n <= 112); 2, 3 cooperative groups of CTAs with 32- and 64-row tiles.
+ * Groups need a workspace of vqc_sp2_purify_workspace bytes (256-byte
+ * aligned, contents undefined); error receives 31 if a group's barrier
+ * expires (it is not written otherwise; the caller zeroes it).
+ */
+int vqc_sp2_purify_workspace(int32_t nmol, int32_t n, int32_t path, uint64_t* bytes);
+int vqc_sp2_purify(const double* fo, int32_t nmol, int32_t n, double nocc, double tol,
+                   int32_t max_steps, int32_t path, double* out, void* work, uint64_t work_bytes,
+                   int32_t* error, void* stream);
+
+/*
  * Mixed-precision J/K over the FP32 whitened tensor stored aux-major per AO
  * row: b_aux_major[mol][mu][Q][nu], row length ld_ao >= nao (ld_ao % 4 == 0;
  * the Coulomb and fitted-density kernels take ld_ao <= 512,

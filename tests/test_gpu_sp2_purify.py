@@ -1,0 +1,66 @@
+"""One-launch FP64 purification against eigenvectors, over the forms' edges.
+
+Sizes sit at the edges of the 8-, 16-, 32- and 64-row tiles, of the 32-column
+K stages and of the one-CTA form; batches at one molecule, several groups and
+more molecules than resident groups.
+"""
+
+import pytest
+import torch
+
+from vibeqc_b200 import _lib
+from vibeqc_b200.scf import _purify_fp64, purify_sp2
+
+pytestmark = pytest.mark.gpu
+
+
+def _fock(nb, n, nocc, seed):
+    """Symmetric matrices with a gap of 0.6 in a spectrum of width about 25, as a Fock matrix has."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rnd = dict(generator=g, dtype=torch.float64, device="cuda")
+    q = torch.linalg.qr(torch.randn(nb, n, n, **rnd))[0]
+    lam = torch.cat([-0.5 - 20.0 * torch.rand(nb, nocc, **rnd) ** 3,
+                     0.1 + 4.0 * torch.rand(nb, n - nocc, **rnd)], dim=1)
+    f = (q * lam[:, None, :]) @ q.transpose(1, 2)
+    v = q[:, :, :nocc]
+    return 0.5 * (f + f.transpose(1, 2)), v @ v.transpose(1, 2)
+
+
+@pytest.mark.parametrize("path,nb,n", [
+    (1, 1, 2), (1, 3, 7), (1, 2, 8), (1, 5, 17), (1, 200, 24), (1, 2, 64), (1, 2, 105), (1, 1, 112),
+    (2, 1, 2), (2, 1, 31), (2, 3, 33), (2, 2, 65), (2, 1, 96), (2, 700, 40), (2, 2, 257),
+    (3, 1, 5), (3, 1, 64), (3, 2, 63), (3, 3, 129), (3, 400, 70), (3, 2, 384), (0, 2, 64), (0, 2, 66),
+    (0, 1, 700)])
+def test_projector_matches_eigenvectors(path, nb, n):
+    nocc = max(1, n // 5)
+    f, want = _fock(nb, n, nocc, 100 * n + nb)
+    got = _purify_fp64(f, nocc, 96, 1e-11, path)
+    # X is idempotent to tr X - tr X^2 < 1e-11 and commutes with F to rounding:
+    # eigenvector error <= n eps |F| / gap = 700 * 2.2e-16 * 25 / 0.6 < 7e-12
+    assert (got - want).abs().max().item() < 2e-11
+    assert torch.equal(got, got.transpose(1, 2))
+
+
+@pytest.mark.parametrize("path,n", [(1, 30), (2, 80), (3, 80)])
+def test_step_cap_and_occupations(path, n):
+    f, _ = _fock(2, n, 4, n)
+    # no step: X is the mapped matrix, whose eigenvalues lie in [0, 1]
+    x0 = torch.linalg.eigvalsh(_purify_fp64(f, 4, 0, 1e-11, path))
+    assert x0.min().item() > -1e-12 and x0.max().item() < 1 + 1e-12
+    # nothing occupied, everything occupied
+    assert _purify_fp64(f, 0, 96, 1e-11, path).abs().max().item() < 1e-11
+    eye = torch.eye(n, dtype=torch.float64, device="cuda")
+    assert (_purify_fp64(f, n, 96, 1e-11, path) - eye).abs().max().item() < 1e-11
+    # non-finite input stays visible and leaves the neighbours alone
+    bad = f.clone()
+    bad[1, 3, 5] = float("nan")
+    got = _purify_fp64(bad, 4, 96, 1e-11, path)
+    assert torch.isnan(got[1]).any() and torch.equal(got[0], _purify_fp64(f[:1], 4, 96, 1e-11, path)[0])
+
+
+def test_layouts_and_arguments():
+    f, want = _fock(3, 48, 9, 1)
+    strided = f.repeat_interleave(2, dim=2)[:, :, ::2]
+    assert (purify_sp2(strided, 9) - want).abs().max().item() < 2e-11
+    with pytest.raises(_lib.VqcError):
+        _purify_fp64(_fock(1, 113, 9, 1)[0], 9, 96, 1e-11, 1)

@@ -120,6 +120,11 @@ _SIGNATURES = {
                         ctypes.c_int64, ctypes.c_int64, _P, _P], ctypes.c_int),
     "vqc_sp2_update": ([_P, _P, _P, ctypes.c_int32, ctypes.c_int32, ctypes.c_double,
                         ctypes.c_double, _P, _P], ctypes.c_int),
+    "vqc_sp2_purify_workspace": ([ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
+                                  ctypes.POINTER(ctypes.c_uint64)], ctypes.c_int),
+    "vqc_sp2_purify": ([_P, ctypes.c_int32, ctypes.c_int32, ctypes.c_double, ctypes.c_double,
+                        ctypes.c_int32, ctypes.c_int32, _P, _P, ctypes.c_uint64, _P, _P],
+                       ctypes.c_int),
     "vqc_unpack_aux_major": ([_P, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                               ctypes.c_int32, _P, _P], ctypes.c_int),
     "vqc_split_tf32": ([_P, _P, _P, ctypes.c_int64, _P], ctypes.c_int),

@@ -16,6 +16,7 @@ rms(dD) < density_tolerance and max|FDS - SDF| <= min(1e-8, density_tolerance)
 
 from __future__ import annotations
 
+import ctypes
 import os
 
 import math
@@ -221,26 +222,23 @@ class _SP2Graph:
 
     The iterate lives in static buffers; converged molecules are copied
     unchanged by the update kernel, so extra steps are harmless and the host
-    reads the device flags once per replay.  ``gemm`` selects how X^2 is
-    formed: "fp64" (batched DGEMM) or "int8" (FP64-accurate products of
-    SP2_SLICES 7-bit slices on the int8 tensor cores, vqc_ozaki_slice_rows +
-    vqc_ozaki_gemm; X is symmetric, so X X^T = X^2, and the sliced product is
-    exactly symmetric because both operands carry the same slices).
+    reads the device flags once per replay.  X^2 is an FP64-accurate product
+    of SP2_SLICES 7-bit slices on the int8 tensor cores
+    (vqc_ozaki_slice_rows + vqc_ozaki_gemm; X is symmetric, so X X^T = X^2,
+    and the sliced product is exactly symmetric because both operands carry
+    the same slices).
     """
 
-    def __init__(self, nb: int, n: int, nocc: int, tol: float, device, steps: int = SP2_GRAPH_STEPS,
-                 gemm: str = "fp64"):
+    def __init__(self, nb: int, n: int, nocc: int, tol: float, device, steps: int = SP2_GRAPH_STEPS):
         self.steps = int(steps)
-        self.gemm = gemm
         self.x = torch.zeros(nb, n, n, dtype=torch.float64, device=device)
         self.x2 = torch.empty_like(self.x)
         self.xn = torch.empty_like(self.x)
         self.done = torch.zeros(nb, dtype=torch.int32, device=device)
         self.err = torch.zeros(1, dtype=torch.int32, device=device)
-        if gemm == "int8":
-            self.ldk = (n + 15) // 16 * 16
-            self.sl = torch.zeros(nb * SP2_SLICES * n * self.ldk, dtype=torch.int8, device=device)
-            self.ex = torch.zeros(nb * n, dtype=torch.int32, device=device)
+        self.ldk = (n + 15) // 16 * 16
+        self.sl = torch.zeros(nb * SP2_SLICES * n * self.ldk, dtype=torch.int8, device=device)
+        self.ex = torch.zeros(nb * n, dtype=torch.int32, device=device)
         self.args = (nb, n, float(nocc), float(tol))
         self.graph = None
         if os.environ.get("VQC_SP2_GRAPHS", "1") == "0":
@@ -263,15 +261,12 @@ class _SP2Graph:
         """``steps`` steps: one graph replay, or eager launches."""
         if self.graph is not None:
             self.graph.replay()
-            GRAPH_LAUNCHES[0] += self.steps * (3 if self.gemm == "int8" else 1)
+            GRAPH_LAUNCHES[0] += self.steps * 3
         else:
             self._steps()
 
     def _square(self, x):
         nb, n = self.args[0], self.args[1]
-        if self.gemm != "int8":
-            torch.bmm(x, x, out=self.x2)
-            return
         st = torch.cuda.current_stream().cuda_stream
         _lib.call("vqc_ozaki_slice_rows", x.data_ptr(), nb, n, n, n, n * n, None, SP2_SLICES,
                   self.sl.data_ptr(), self.ldk, self.ex.data_ptr(), st)
@@ -305,21 +300,23 @@ def purify_sp2(fo: torch.Tensor, nocc: int, max_steps: int = 96, tol: float = 1e
     Second-order spectral projection (Niklasson, Phys. Rev. B 66, 155115
     (2002)): map the spectrum into [0, 1] with Gershgorin bounds, then apply
     X <- X^2 or X <- 2X - X^2, whichever moves tr X toward ``nocc``, until
-    tr(X) - tr(X^2) < tol.  Per step: one batched GEMM and one native update
-    kernel (vqc_sp2_update); convergence flags stay on the device.  Steps run
-    in CUDA graphs of SP2_GRAPH_STEPS (cached in ``graphs``, one per shape and
-    tolerance), and the flags are read once per graph replay.  ``steps`` (even)
-    is the number of steps per graph and ``gemm`` the X^2 product ("fp64"
-    DGEMM or "int8" sliced tensor-core products), both autotuned schedule
-    choices.
+    tr(X) - tr(X^2) < tol.  With ``gemm="fp64"`` the whole purification is one
+    native launch (vqc_sp2_purify).  ``gemm="int8"`` forms X^2 from sliced
+    tensor-core products, in CUDA graphs of ``steps`` (even) steps cached in
+    ``graphs``, one per shape and tolerance; the convergence flags stay on the
+    device and are read once per graph replay.
     """
     nb, n, _ = fo.shape
+    # the cap counts whole groups of ``steps``, as the graphs run them
+    cap = -(-max_steps // int(steps)) * int(steps)
+    if gemm != "int8":
+        return _purify_fp64(fo, nocc, cap, tol)
     diag = torch.diagonal(fo, dim1=1, dim2=2)
     radius = fo.abs().sum(dim=2) - diag.abs()
     emin = (diag - radius).min(dim=1).values
     emax = (diag + radius).max(dim=1).values
     eye = torch.eye(n, dtype=fo.dtype, device=fo.device)
-    key = (nb, n, int(nocc), float(tol), str(fo.device), int(steps), gemm)
+    key = (nb, n, int(nocc), float(tol), str(fo.device), int(steps))
     if graphs is None:
         graphs = {}
     g = graphs.get(key)
@@ -327,16 +324,34 @@ def purify_sp2(fo: torch.Tensor, nocc: int, max_steps: int = 96, tol: float = 1e
         held = sum(3 * v.x.numel() * 8 for v in graphs.values())
         if held + 3 * nb * n * n * 8 > SP2_GRAPH_CACHE_BYTES:
             graphs.clear()
-        g = graphs[key] = _SP2Graph(nb, n, nocc, tol, fo.device, steps, gemm)
+        g = graphs[key] = _SP2Graph(nb, n, nocc, tol, fo.device, steps)
     torch.div(emax[:, None, None] * eye - fo, (emax - emin)[:, None, None], out=g.x)
     g.done.zero_()
-    for _ in range(0, max_steps, int(steps)):
+    for _ in range(0, cap, int(steps)):
         g.run()
         if bool(g.done.all()):
             break
-    if gemm == "int8" and int(g.err.item()) != 0:
+    if int(g.err.item()) != 0:
         raise _lib.VqcError(6, f"tensor-core purification wait expired (code {int(g.err.item())})")
     return 0.5 * (g.x + g.x.transpose(1, 2))
+
+
+def _purify_fp64(fo: torch.Tensor, nocc: int, max_steps: int, tol: float,
+                 path: int = 0) -> torch.Tensor:
+    """purify_sp2 as one native launch; ``path`` as in vqc_sp2_purify."""
+    nb, n, _ = fo.shape
+    fo = fo.to(torch.float64).contiguous()
+    out = torch.empty_like(fo)
+    need = ctypes.c_uint64()
+    _lib.call("vqc_sp2_purify_workspace", nb, n, path, ctypes.byref(need))
+    work = torch.empty(need.value, dtype=torch.uint8, device=fo.device)
+    err = torch.zeros(1, dtype=torch.int32, device=fo.device)
+    _lib.call("vqc_sp2_purify", fo.data_ptr(), nb, n, float(nocc), float(tol), max_steps, path,
+              out.data_ptr(), work.data_ptr(), need.value, err.data_ptr(), _stream_ptr())
+    # only the groups' barriers can fail; one CTA per molecule waits for nothing
+    if need.value and int(err.item()) != 0:
+        raise _lib.VqcError(6, f"purification wait expired (code {int(err.item())})")
+    return out
 
 
 def _cholqr2(y: torch.Tensor):

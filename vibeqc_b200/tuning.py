@@ -12,11 +12,12 @@ the device that will run them and stored in a table
   FP64-accurate B; small shapes can favour the plain GEMMs;
 * ``gram_waves``: the exchange Gram product splits its K range until about
   this many CTAs per SM exist (library knob ``VQC_TUNE_GRAM_WAVES``);
-* ``sp2_steps``: purification steps per captured CUDA graph (more steps mean
-  fewer host round trips, but converged molecules idle longer);
-* ``sp2_gemm``: how the mixed path forms the purification product X^2 --
-  batched FP64 GEMMs (``"fp64"``) or FP64-accurate sliced products on the
-  int8 tensor cores (``"int8"``).
+* ``sp2_steps``: purification steps per captured CUDA graph of the sliced
+  products (more steps mean fewer host round trips, but converged molecules
+  idle longer); the FP64 purification is one launch and has no graphs;
+* ``sp2_gemm``: how the mixed path purifies -- on the FP64 tensor pipe in one
+  launch (``"fp64"``) or with FP64-accurate sliced products on the int8 tensor
+  cores (``"int8"``).
 
     python -m vibeqc_b200.tuning [--count 256] [--out path]
 
@@ -194,7 +195,8 @@ def tune_chunk(chunk, xyz) -> tuple[Schedule, dict]:
     for n_steps in SP2_STEPS:
         graphs: dict = {}
         timings["sp2_steps"][str(n_steps)] = round(
-            _time(lambda: purify_sp2(fo, chunk.nocc, graphs=graphs, steps=n_steps)), 3)
+            _time(lambda: purify_sp2(fo, chunk.nocc, graphs=graphs, steps=n_steps,
+                                     gemm="int8")), 3)
     steps_best = int(min(timings["sp2_steps"], key=timings["sp2_steps"].get))
     timings["sp2_gemm"] = {}
     for gemm in SP2_GEMMS:
