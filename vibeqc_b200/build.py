@@ -55,26 +55,24 @@ def gen_sph_table() -> Path:
     return out
 
 
-def _generator_grid() -> tuple[str, str]:
-    """(DEG, H) as written in gen_rys_table.py."""
-    deg = h = ""
+def _generator_grid() -> dict[str, str]:
+    """LAYOUT, DEG and H as written in gen_rys_table.py."""
+    grid = {}
     for line in (CSRC / "gen_rys_table.py").read_text().splitlines():
-        if line.startswith("DEG ="):
-            deg = line.split("=")[1].split("#")[0].strip()
-        elif line.startswith("H ="):
-            h = line.split("=")[1].split("#")[0].strip()
-    return deg, h
+        name, _, value = line.partition(" = ")
+        if name in ("LAYOUT", "DEG", "H"):
+            grid[name] = value.split("#")[0].strip()
+    return grid
 
 
 def ensure_rys_table() -> Path:
-    """Generate rys_table.inc when missing or written for another (DEG, H) grid."""
+    """Generate rys_table.inc when missing or written for another grid or layout."""
     out = CSRC / "rys_table.inc"
-    deg, h = _generator_grid()
     stale = True
     if out.exists():
         head = out.read_text()[:2000]
-        stale = (f"#define RYS_DEG {deg}\n" not in head
-                 or f"#define RYS_H {float(h)!r}\n" not in head)
+        stale = any(f"#define RYS_{name} {value}\n" not in head
+                    for name, value in _generator_grid().items())
     if stale:
         subprocess.run([sys.executable, str(CSRC / "gen_rys_table.py")], check=True)
     return out

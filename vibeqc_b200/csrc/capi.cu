@@ -194,7 +194,7 @@ int Plan::build(const vqc_batch_desc& d) {
     if ((st = upload(owned, pl2[c], &dpairs2[c]))) return st;
   }
   auto add_class = [&](std::vector<ClassLaunch>& list, int la, int lb, int lc, const int2* pairs,
-                       std::vector<ClassMol>& cms, int per_block) -> int {
+                       std::vector<ClassMol>& cms, int per_block, int nab = 0) -> int {
     if (cms.empty()) return VQC_STATUS_SUCCESS;
     int nb = 0;
     for (auto& c : cms) {
@@ -206,7 +206,7 @@ int Plan::build(const vqc_batch_desc& d) {
     ClassMol* dcm = nullptr;
     int s2 = upload(owned, cms, &dcm);
     if (s2) return s2;
-    list.push_back(ClassLaunch{la, lb, lc, pairs, dcm, (int)cms.size(), nb});
+    list.push_back(ClassLaunch{la, lb, lc, nab, pairs, dcm, (int)cms.size(), nb});
     return VQC_STATUS_SUCCESS;
   };
   for (int la = 0; la <= kMaxKernelL; ++la)
@@ -215,6 +215,8 @@ int Plan::build(const vqc_batch_desc& d) {
       std::vector<ClassMol> one;
       for (int m = 0; m < nmol; ++m)
         if (pcnt[c][m]) one.push_back(ClassMol{m, pbeg[c][m], 0, 0, pcnt[c][m], 0});
+      int nab = 1;
+      for (const int2& pr : pl[c]) nab = std::max(nab, orb_h.nprim[pr.x] * orb_h.nprim[pr.y]);
       if ((st = add_class(cls1e, la, lb, 0, dpairs[c], one, 128))) return st;
       for (int lc = 0; lc <= kMaxKernelL; ++lc) {
         std::vector<ClassMol> cm3;
@@ -224,7 +226,7 @@ int Plan::build(const vqc_batch_desc& d) {
           if (tri > 0x7fffffffLL) return fail(VQC_STATUS_INVALID_ARGUMENT, "molecule too large for the 3-centre work list");
           cm3.push_back(ClassMol{m, pbeg[c][m], abeg[lc][m], acnt[lc][m], (int)tri, 0});
         }
-        if ((st = add_class(cls3c, la, lb, lc, dpairs[c], cm3, slots3c(la, lb, lc, sph)))) return st;
+        if ((st = add_class(cls3c, la, lb, lc, dpairs[c], cm3, slots3c(la, lb, lc, sph), nab))) return st;
         if (!cm3.empty()) cls3c_host.push_back(cm3);
       }
       std::vector<ClassMol> cm2;

@@ -9,8 +9,12 @@ For every n <= NMAX this script computes (u_i, w_i) in 80-digit arithmetic:
 moments F_k(T) = 1F1(k+1/2; k+3/2; -T) / (2k+1), the three-term recurrence by
 Gautschi's Chebyshev algorithm, and the Golub-Welsch eigenproblem of the Jacobi
 matrix.  On [0, T_asym(n)) it fits each u_i(T) and w_i(T) with a Chebyshev
-series of degree DEG on intervals of width H (nodes at Chebyshev points), and
-writes the coefficients as hex doubles into ``rys_table.inc``.  For
+series of degree DEG on intervals of width H (nodes at Chebyshev points),
+expands the series in powers of x in [-1, 1] (still in 80 digits; the series
+falls so fast that the powers lose nothing) and writes the coefficients as hex
+doubles into ``rys_table.inc``: per interval and root, from the highest power
+down, (u, w) coefficient pairs, so that a Horner step of both takes one 16-byte
+load.  For
 T >= T_asym(n) the kernels use the large-T limit u_i = x_i^2 / T,
 w_i = W_i / sqrt(T) with (x_i, W_i) the positive Gauss-Hermite nodes/weights of
 order 2n; those constants are written too.  T_asym(n) is the smallest grid
@@ -29,7 +33,8 @@ from pathlib import Path
 import mpmath as mp
 
 NMAX = 7
-DEG = 9           # Chebyshev degree per interval
+LAYOUT = 2        # version of the coefficients' form and order in the table
+DEG = 9           # polynomial degree per interval
 H = 0.5           # interval width in T
 DPS = 80
 TOL_ASYM = 1e-15
@@ -109,16 +114,31 @@ def fit_interval(args):
             c *= mp.mpf(2) / (DEG + 1)
             if jdeg == 0:
                 c /= 2
-            row.append(float(c))
-        coefs.append(row)
+            row.append(c)
+        coefs.append([float(v) for v in powers(row)])
     return coefs
 
 
-def clenshaw(c, x):
-    b1 = b2 = 0.0
-    for k in range(len(c) - 1, 0, -1):
-        b1, b2 = 2 * x * b1 - b2 + c[k], b1
-    return x * b1 - b2 + c[0]
+def powers(cheb):
+    """Coefficients of x^0, x^1, ... of sum_k cheb[k] T_k(x)."""
+    n = len(cheb)
+    prev, cur = [mp.mpf(1)], [mp.mpf(0), mp.mpf(1)]
+    out = [mp.mpf(0)] * n
+    for k in range(n):
+        for i, t in enumerate(prev):
+            out[i] += cheb[k] * t
+        nxt = [mp.mpf(0)] + [2 * t for t in cur]
+        for i, t in enumerate(prev):
+            nxt[i] -= t
+        prev, cur = cur, nxt
+    return out
+
+
+def horner(c, x):
+    v = c[-1]
+    for k in range(len(c) - 2, -1, -1):
+        v = v * x + c[k]
+    return v
 
 
 def t_asym(n, xs, ws):
@@ -164,16 +184,17 @@ def main():
             x = 2 * (t - i * H) / H - 1
             ue, we = rys_exact(n, mp.mpf(t))
             ref = [float(v) for v in ue + we]
-            got = [clenshaw(c, x) for c in table[n][i]]
+            got = [horner(c, x) for c in table[n][i]]
             err = max(err, max(abs(g - r) / abs(r) for g, r in zip(got, ref)))
         worst[n] = err
     print("max relative fit error per n:", worst, flush=True)
     lines = [
-        "// Generated by gen_rys_table.py -- Rys nodes/weights as Chebyshev series.",
+        "// Generated by gen_rys_table.py -- Rys nodes/weights as polynomials on intervals.",
         f"// NMAX={NMAX} DEG={DEG} H={H}; max relative fit error per n: "
         + ", ".join(f"{n}:{worst[n]:.1e}" for n in worst),
         "// Included by vqc_internal.cuh inside namespace vqc (device code only).",
         f"#define RYS_NMAX {NMAX}",
+        f"#define RYS_LAYOUT {LAYOUT}",
         f"#define RYS_DEG {DEG}",
         f"#define RYS_H {H!r}",
         "template <int N> struct RysIntervals;",
@@ -191,10 +212,11 @@ def main():
             f"template <> struct RysOffset<{n}> {{ static constexpr int value = {offs[n - 1]}; }};"
         )
     lines.append(f"#define RYS_TABLE_SIZE {total}")
-    lines.append("static __device__ const double d_rys_table[RYS_TABLE_SIZE] = {")
+    lines.append("static __device__ __align__(32) const double d_rys_table[RYS_TABLE_SIZE] = {")
     for n in range(1, NMAX + 1):
         for c in table[n]:
-            for row in c:
+            for r in range(n):
+                row = [v for k in range(DEG, -1, -1) for v in (c[r][k], c[n + r][k])]
                 lines.append(",".join(float.hex(v) for v in row) + ",")
     lines.append("};")
     # asymptotic constants: x_i^2 and W_i, [n][i] padded to NMAX

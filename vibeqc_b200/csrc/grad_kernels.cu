@@ -32,15 +32,6 @@ __device__ __forceinline__ void cart_of_g(int l, int k, int& x, int& y, int& z) 
   z = rem;
 }
 
-__device__ __forceinline__ int find_cm_g(const ClassMol* __restrict__ cms, int ncm, int block) {
-  int lo = 0, hi = ncm - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (cms[mid].chunk_begin <= block) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
 // Add v (3 components) to grad[3*key+d] across a full warp, segmented by runs
 // of equal key in lane order; key < 0 contributes nothing.
 __device__ __forceinline__ void warp_seg_add(double* __restrict__ grad, int key, double vx,
@@ -100,9 +91,31 @@ __device__ __forceinline__ void weights_to_cart(int mode, const double (&w)[NOA]
     }
 }
 
-}  // namespace
+// gA, gB += ww * d/dA, d/dB of one Cartesian product x y z of 2-D factors
+// I[i][j] raised by one in both indices; a2 = 2a, b2 = 2b.  (Component indices
+// are compile-time constants in every caller.)
+template <int MA, int MB>
+__device__ __forceinline__ void contract_derivative(const double (&ix)[MA][MB], const double (&iy)[MA][MB],
+                                                    const double (&iz)[MA][MB], int ax, int ay, int az,
+                                                    int bx, int by, int bz, double a2, double b2, double ww,
+                                                    double (&gA)[3], double (&gB)[3]) {
+  const double x0 = ix[ax][bx], y0 = iy[ay][by], z0 = iz[az][bz];
+  const double dax = a2 * ix[ax + 1][bx] - (ax ? ax * ix[ax ? ax - 1 : 0][bx] : 0.0);
+  const double day = a2 * iy[ay + 1][by] - (ay ? ay * iy[ay ? ay - 1 : 0][by] : 0.0);
+  const double daz = a2 * iz[az + 1][bz] - (az ? az * iz[az ? az - 1 : 0][bz] : 0.0);
+  const double dbx = b2 * ix[ax][bx + 1] - (bx ? bx * ix[ax][bx ? bx - 1 : 0] : 0.0);
+  const double dby = b2 * iy[ay][by + 1] - (by ? by * iy[ay][by ? by - 1 : 0] : 0.0);
+  const double dbz = b2 * iz[az][bz + 1] - (bz ? bz * iz[az][bz ? bz - 1 : 0] : 0.0);
+  const double wx0 = ww * x0, wyz = ww * y0 * z0, wy = wx0 * z0, wz = wx0 * y0;
+  gA[0] = fma(wyz, dax, gA[0]);
+  gA[1] = fma(wy, day, gA[1]);
+  gA[2] = fma(wz, daz, gA[2]);
+  gB[0] = fma(wyz, dbx, gB[0]);
+  gB[1] = fma(wy, dby, gB[1]);
+  gB[2] = fma(wz, dbz, gB[2]);
+}
 
-__host__ __device__ constexpr int round32(int n) { return (n + 31) / 32 * 32; }
+}  // namespace
 
 // ---------------------------------------------------------------------------
 // 3-centre derivative contraction
@@ -113,7 +126,7 @@ __global__ void __launch_bounds__(round32(Int3cCfg<LA, LB, LC, SPH>::THREADS),
                                   min_ctas_grad3c(LA, LB, LC))
     grad3c_kernel(DevBasis orb, DevBasis aux, const double* __restrict__ xyz,
                   const DevMol* __restrict__ mols, const int2* __restrict__ pairs,
-                  const ClassMol* __restrict__ cms, int ncm, const double* __restrict__ abar,
+                  const ClassMol* __restrict__ cms, int ncm, int stride, const double* __restrict__ abar,
                   double* __restrict__ grad) {
   using C = Int3cCfg<LA, LB, LC, SPH>;
   constexpr int NCA = ncart(LA), NCB = ncart(LB), NCC = ncart(LC);
@@ -123,105 +136,87 @@ __global__ void __launch_bounds__(round32(Int3cCfg<LA, LB, LC, SPH>::THREADS),
   constexpr Cart<LA> ca{};
   constexpr Cart<LB> cb{};
 
-  const ClassMol cm = cms[find_cm_g(cms, ncm, blockIdx.x)];
+  const ClassMol cm = cms[find_cm(cms, ncm, blockIdx.x)];
   const int t0 = (blockIdx.x - cm.chunk_begin) * C::SLOTS;
   const int slot = threadIdx.x / NCC, kc = threadIdx.x % NCC;
   const int t = t0 + slot;
   const bool valid = slot < C::SLOTS && t < cm.ntriples;
+  const int q0 = t0 / cm.naux;
+  const int npairs = (min(t0 + C::SLOTS, cm.ntriples) - 1) / cm.naux - q0 + 1;
+  const int2* cpairs = pairs + cm.pair_begin + q0;
+  __shared__ __align__(16) PairTable tab;
   double gA[3] = {0.0, 0.0, 0.0}, gB[3] = {0.0, 0.0, 0.0};
   int atomA = -1, atomB = -1, atomC = -1;
+  int2 pr = make_int2(0, 0);
+  int sc = 0, kx = 0, ky = 0, kz = 0;
+  bool work = false;
+  double wc[NCA][NCB] = {};
   if (valid) {
-    const int2 pr = pairs[cm.pair_begin + t / cm.naux];
-    const int sc = cm.aux_begin + t % cm.naux;
+    pr = cpairs[t / cm.naux - q0];
+    sc = cm.aux_begin + t % cm.naux;
     atomA = orb.atom[pr.x];
     atomB = orb.atom[pr.y];
     atomC = aux.atom[sc];
-    if (!(atomA == atomB && atomB == atomC)) {
-      const DevMol mol = mols[cm.mol];
-      int kx, ky, kz;
-      cart_of_g(LC, kc, kx, ky, kz);
-      // weights: Abar block for this Cartesian aux component, in Cartesian a, b
-      double wsph[NOA][NOB];
-      const int fa = orb.func_off[pr.x], fb = orb.func_off[pr.y], fc = aux.func_off[sc];
+    work = !(atomA == atomB && atomB == atomC);
+  }
+  Triple tri;
+  if (work) tri.load(orb, aux, xyz, pr, sc);
+  if (work) {
+    const DevMol mol = mols[cm.mol];
+    cart_of_g(LC, kc, kx, ky, kz);
+    // weights: Abar block for this Cartesian aux component, in Cartesian a, b
+    double wsph[NOA][NOB];
+    const int fa = orb.func_off[pr.x], fb = orb.func_off[pr.y], fc = aux.func_off[sc];
 #pragma unroll
-      for (int i = 0; i < NOA; ++i)
+    for (int i = 0; i < NOA; ++i)
 #pragma unroll
-        for (int j = 0; j < NOB; ++j) {
-          const long long mu = fa + i, nu = fb + j;
-          const long long hi = mu > nu ? mu : nu, lo = mu > nu ? nu : mu;
-          const double* row = abar + mol.a_off + (hi * (hi + 1) / 2 + lo) * mol.naux + fc;
-          double s = 0.0;
+      for (int j = 0; j < NOB; ++j) {
+        const long long mu = fa + i, nu = fb + j;
+        const long long hi = mu > nu ? mu : nu, lo = mu > nu ? nu : mu;
+        const double* row = abar + mol.a_off + (hi * (hi + 1) / 2 + lo) * mol.naux + fc;
+        double s = 0.0;
 #pragma unroll
-          for (int k = 0; k < NOC; ++k) s = fma(c_trans[MODE][LC][k][kc], __ldg(row + k), s);
-          wsph[i][j] = s;
-        }
-      double wc[NCA][NCB];
-      weights_to_cart<LA, LB, NOA, NOB>(MODE, wsph, wc);
-      const double pair_factor = (pr.x == pr.y) ? 1.0 : 2.0;
-      const double* A = xyz + 3 * atomA;
-      const double* B = xyz + 3 * atomB;
-      const double* Cc = xyz + 3 * atomC;
-      const double ab[3] = {A[0] - B[0], A[1] - B[1], A[2] - B[2]};
-      const double rab2 = ab[0] * ab[0] + ab[1] * ab[1] + ab[2] * ab[2];
-      const int pa0 = orb.prim_off[pr.x], na = orb.nprim[pr.x];
-      const int pb0 = orb.prim_off[pr.y], nb = orb.nprim[pr.y];
-      const int pc0 = aux.prim_off[sc], nc = aux.nprim[sc];
-      for (int ia = 0; ia < na; ++ia) {
-        const double a = orb.exps[pa0 + ia], ca_ = orb.coefs[pa0 + ia];
-        for (int ib = 0; ib < nb; ++ib) {
-          const double b = orb.exps[pb0 + ib], cb_ = orb.coefs[pb0 + ib];
-          const double p = a + b, ip = 1.0 / p;
-          const double kab = exp(-a * b * ip * rab2) * ca_ * cb_;
-          if (fabs(kab) < kPrimPairCut) continue;
-          const double P[3] = {(a * A[0] + b * B[0]) * ip, (a * A[1] + b * B[1]) * ip,
-                               (a * A[2] + b * B[2]) * ip};
-          for (int ic = 0; ic < nc; ++ic) {
-            const double g = aux.exps[pc0 + ic], cg = aux.coefs[pc0 + ic];
-            const double pq = p + g, ipq = 1.0 / pq;
-            const double PQ[3] = {P[0] - Cc[0], P[1] - Cc[1], P[2] - Cc[2]};
-            const double tt = p * g * ipq * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
-            const double pref =
-                2.0 * kPi * kPi * sqrt(kPi) * ip / g * sqrt(ipq) * kab * cg * pair_factor;
-            double u[NR], w[NR];
-            rys_roots<NR>(tt, u, w);
+        for (int k = 0; k < NOC; ++k) s = fma(c_trans[MODE][LC][k][kc], __ldg(row + k), s);
+        wsph[i][j] = s;
+      }
+    weights_to_cart<LA, LB, NOA, NOB>(MODE, wsph, wc);
+  }
+  for_prim_pairs(tab, orb, xyz, cpairs, npairs, stride, t / cm.naux - q0, tri.nab,
+                 [&](const PrimPair* e0, const PrimPair* e1) {
+    const double pair_factor = (pr.x == pr.y) ? 1.0 : 2.0;
+    for (int ic = 0; ic < tri.nc; ++ic) {
+      const double g = ic ? aux.exps[tri.pc0 + ic] : tri.g0, hg = 0.5 / g;
+      const double cg = 2.0 * hg * (ic ? aux.coefs[tri.pc0 + ic] : tri.c0) * pair_factor;
+      for (const PrimPair* e = e0; e < e1; ++e) {
+        const double kab = e->k;
+        if (kab == 0.0) continue;
+        const double p = e->p, hip = e->hip, ipq = 1.0 / (p + g), a2 = e->a2, b2 = e->b2;
+        const double P[3] = {e->x, e->y, e->z};
+        const double PQ[3] = {P[0] - tri.C[0], P[1] - tri.C[1], P[2] - tri.C[2]};
+        const double tt = p * g * ipq * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
+        const double pref = sqrt(ipq) * kab * cg;
+        double u[NR], w[NR];
+        rys_roots<NR>(tt, u, w);
 #pragma unroll
-            for (int r = 0; r < NR; ++r) {
-              const double ur = u[r];
-              const double qf = g * ipq * ur, pf = p * ipq * ur;
-              const double b00 = 0.5 * ipq * ur, b10 = 0.5 * ip * (1.0 - qf),
-                           b01 = 0.5 / g * (1.0 - pf);
-              double ix[LA + 2][LB + 2], iy[LA + 2][LB + 2], iz[LA + 2][LB + 2];
-              rys_2d<LA + 1, LB + 1, LC>(P[0] - A[0] - qf * PQ[0], pf * PQ[0], b10, b01, b00, ab[0], kx, ix);
-              rys_2d<LA + 1, LB + 1, LC>(P[1] - A[1] - qf * PQ[1], pf * PQ[1], b10, b01, b00, ab[1], ky, iy);
-              rys_2d<LA + 1, LB + 1, LC>(P[2] - A[2] - qf * PQ[2], pf * PQ[2], b10, b01, b00, ab[2], kz, iz);
-              const double wr = pref * w[r];
+        for (int r = 0; r < NR; ++r) {
+          const double ur = ipq * u[r];
+          const double qf = g * ur, pf = p * ur;
+          const double b00 = 0.5 * ur, b10 = fma(-hip, qf, hip), b01 = fma(-hg, pf, hg);
+          double ix[LA + 2][LB + 2], iy[LA + 2][LB + 2], iz[LA + 2][LB + 2];
+          rys_2d<LA + 1, LB + 1, LC>(P[0] - tri.A[0] - qf * PQ[0], pf * PQ[0], b10, b01, b00, tri.ab[0], kx, ix);
+          rys_2d<LA + 1, LB + 1, LC>(P[1] - tri.A[1] - qf * PQ[1], pf * PQ[1], b10, b01, b00, tri.ab[1], ky, iy);
+          rys_2d<LA + 1, LB + 1, LC>(P[2] - tri.A[2] - qf * PQ[2], pf * PQ[2], b10, b01, b00, tri.ab[2], kz, iz);
+          const double wr = pref * w[r];
 #pragma unroll
-              for (int i = 0; i < NCA; ++i)
+          for (int i = 0; i < NCA; ++i)
 #pragma unroll
-                for (int j = 0; j < NCB; ++j) {
-                  const int ax = ca.x[i], ay = ca.y[i], az = ca.z[i];
-                  const int bx = cb.x[j], by = cb.y[j], bz = cb.z[j];
-                  const double x0 = ix[ax][bx], y0 = iy[ay][by], z0 = iz[az][bz];
-                  const double dax = 2.0 * a * ix[ax + 1][bx] - (ax ? ax * ix[ax ? ax - 1 : 0][bx] : 0.0);
-                  const double day = 2.0 * a * iy[ay + 1][by] - (ay ? ay * iy[ay ? ay - 1 : 0][by] : 0.0);
-                  const double daz = 2.0 * a * iz[az + 1][bz] - (az ? az * iz[az ? az - 1 : 0][bz] : 0.0);
-                  const double dbx = 2.0 * b * ix[ax][bx + 1] - (bx ? bx * ix[ax][bx ? bx - 1 : 0] : 0.0);
-                  const double dby = 2.0 * b * iy[ay][by + 1] - (by ? by * iy[ay][by ? by - 1 : 0] : 0.0);
-                  const double dbz = 2.0 * b * iz[az][bz + 1] - (bz ? bz * iz[az][bz ? bz - 1 : 0] : 0.0);
-                  const double ww = wr * wc[i][j];
-                  gA[0] = fma(ww, dax * y0 * z0, gA[0]);
-                  gA[1] = fma(ww, x0 * day * z0, gA[1]);
-                  gA[2] = fma(ww, x0 * y0 * daz, gA[2]);
-                  gB[0] = fma(ww, dbx * y0 * z0, gB[0]);
-                  gB[1] = fma(ww, x0 * dby * z0, gB[1]);
-                  gB[2] = fma(ww, x0 * y0 * dbz, gB[2]);
-                }
-            }
-          }
+            for (int j = 0; j < NCB; ++j)
+              contract_derivative(ix, iy, iz, ca.x[i], ca.y[i], ca.z[i], cb.x[j], cb.y[j], cb.z[j], a2,
+                                  b2, wr * wc[i][j], gA, gB);
         }
       }
     }
-  }
+  });
   warp_seg_add(grad, atomA, gA[0], gA[1], gA[2]);
   warp_seg_add(grad, atomB, gB[0], gB[1], gB[2]);
   warp_seg_add(grad, atomC, -(gA[0] + gB[0]), -(gA[1] + gB[1]), -(gA[2] + gB[2]));
@@ -248,10 +243,10 @@ __host__ __device__ constexpr int rp_threads_g3c(int la, int lb, int lc, bool sp
 
 template <int LA, int LB, int LC, bool SPH>
 __global__ void __launch_bounds__(rp_threads_g3c(LA, LB, LC, SPH),
-                                  min_ctas_rp(rp_threads_g3c(LA, LB, LC, SPH)))
+                                  min_ctas_rp(rp_threads_g3c(LA, LB, LC, SPH), LA + LB + LC))
     grad3c_rp_kernel(DevBasis orb, DevBasis aux, const double* __restrict__ xyz,
                      const DevMol* __restrict__ mols, const int2* __restrict__ pairs,
-                     const ClassMol* __restrict__ cms, int ncm, const double* __restrict__ abar,
+                     const ClassMol* __restrict__ cms, int ncm, int stride, const double* __restrict__ abar,
                      double* __restrict__ grad) {
   using C = Int3cCfg<LA, LB, LC, SPH>;
   constexpr int NCA = ncart(LA), NCB = ncart(LB), NCC = ncart(LC);
@@ -263,11 +258,15 @@ __global__ void __launch_bounds__(rp_threads_g3c(LA, LB, LC, SPH),
   constexpr Cart<LB> cb{};
   constexpr Cart<LC> cc{};
 
-  const ClassMol cm = cms[find_cm_g(cms, ncm, blockIdx.x)];
+  const ClassMol cm = cms[find_cm(cms, ncm, blockIdx.x)];
   const int t0 = (blockIdx.x - cm.chunk_begin) * C::SLOTS;
   const int slot = threadIdx.x / NR, r = threadIdx.x % NR;
   const int t = t0 + slot;
   const bool valid = slot < C::SLOTS && t < cm.ntriples;
+  const int q0 = t0 / cm.naux;
+  const int npairs = (min(t0 + C::SLOTS, cm.ntriples) - 1) / cm.naux - q0 + 1;
+  const int2* cpairs = pairs + cm.pair_begin + q0;
+  __shared__ __align__(16) PairTable tab;
   // contraction weights of every Cartesian aux component, Cartesian in a and
   // b: one copy per slot in shared memory, formed by the slot's first root
   // thread and read by all of its roots (a register copy per root thread held
@@ -279,13 +278,15 @@ __global__ void __launch_bounds__(rp_threads_g3c(LA, LB, LC, SPH),
   int sc = 0;
   bool work = false;
   if (valid) {
-    pr = pairs[cm.pair_begin + t / cm.naux];
+    pr = cpairs[t / cm.naux - q0];
     sc = cm.aux_begin + t % cm.naux;
     atomA = orb.atom[pr.x];
     atomB = orb.atom[pr.y];
     atomC = aux.atom[sc];
     work = !(atomA == atomB && atomB == atomC);
   }
+  Triple tri;
+  if (work) tri.load(orb, aux, xyz, pr, sc);
   if (work && r == 0) {
     const DevMol mol = mols[cm.mol];
     const int fa = orb.func_off[pr.x], fb = orb.func_off[pr.y], fc = aux.func_off[sc];
@@ -320,77 +321,47 @@ __global__ void __launch_bounds__(rp_threads_g3c(LA, LB, LC, SPH),
         for (int j = 0; j < NCB; ++j) wsh[slot][(z * NCA + i) * NCB + j] = wcz[i][j];
     }
   }
-  __syncthreads();
-  if (work) {
-    {
-      const double pair_factor = (pr.x == pr.y) ? 1.0 : 2.0;
-      const double* A = xyz + 3 * atomA;
-      const double* B = xyz + 3 * atomB;
-      const double* Cc = xyz + 3 * atomC;
-      const double ab[3] = {A[0] - B[0], A[1] - B[1], A[2] - B[2]};
-      const double rab2 = ab[0] * ab[0] + ab[1] * ab[1] + ab[2] * ab[2];
-      const int pa0 = orb.prim_off[pr.x], na = orb.nprim[pr.x];
-      const int pb0 = orb.prim_off[pr.y], nb = orb.nprim[pr.y];
-      const int pc0 = aux.prim_off[sc], nc = aux.nprim[sc];
-      for (int ia = 0; ia < na; ++ia) {
-        const double a = orb.exps[pa0 + ia], ca_ = orb.coefs[pa0 + ia];
-        for (int ib = 0; ib < nb; ++ib) {
-          const double b = orb.exps[pb0 + ib], cb_ = orb.coefs[pb0 + ib];
-          const double p = a + b, ip = 1.0 / p;
-          const double kab = exp(-a * b * ip * rab2) * ca_ * cb_;
-          if (fabs(kab) < kPrimPairCut) continue;
-          const double P[3] = {(a * A[0] + b * B[0]) * ip, (a * A[1] + b * B[1]) * ip,
-                               (a * A[2] + b * B[2]) * ip};
-          for (int ic = 0; ic < nc; ++ic) {
-            const double g = aux.exps[pc0 + ic], cg = aux.coefs[pc0 + ic];
-            const double pq = p + g, ipq = 1.0 / pq;
-            const double PQ[3] = {P[0] - Cc[0], P[1] - Cc[1], P[2] - Cc[2]};
-            const double tt = p * g * ipq * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
-            const double pref =
-                2.0 * kPi * kPi * sqrt(kPi) * ip / g * sqrt(ipq) * kab * cg * pair_factor;
-            double ur, wr0;
-            rys_root_one<NR>(tt, r, ur, wr0);
-            const double qf = g * ipq * ur, pf = p * ipq * ur;
-            const double b00 = 0.5 * ipq * ur, b10 = 0.5 * ip * (1.0 - qf),
-                         b01 = 0.5 / g * (1.0 - pf);
-            double gx[LAB1 + 1][LC + 1], gy[LAB1 + 1][LC + 1], gz[LAB1 + 1][LC + 1];
-            rys_vrr<LAB1, LC>(P[0] - A[0] - qf * PQ[0], pf * PQ[0], b10, b01, b00, gx);
-            rys_vrr<LAB1, LC>(P[1] - A[1] - qf * PQ[1], pf * PQ[1], b10, b01, b00, gy);
-            rys_vrr<LAB1, LC>(P[2] - A[2] - qf * PQ[2], pf * PQ[2], b10, b01, b00, gz);
-            const double wr = pref * wr0;
+  // (for_prim_pairs synchronises the CTA before any thread reads the weights)
+  for_prim_pairs(tab, orb, xyz, cpairs, npairs, stride, t / cm.naux - q0, tri.nab,
+                 [&](const PrimPair* e0, const PrimPair* e1) {
+    const double pair_factor = (pr.x == pr.y) ? 1.0 : 2.0;
+    for (int ic = 0; ic < tri.nc; ++ic) {
+      const double g = ic ? aux.exps[tri.pc0 + ic] : tri.g0, hg = 0.5 / g;
+      const double cg = 2.0 * hg * (ic ? aux.coefs[tri.pc0 + ic] : tri.c0) * pair_factor;
+      for (const PrimPair* e = e0; e < e1; ++e) {
+        const double kab = e->k;
+        if (kab == 0.0) continue;
+        const double p = e->p, hip = e->hip, ipq = 1.0 / (p + g), a2 = e->a2, b2 = e->b2;
+        const double P[3] = {e->x, e->y, e->z};
+        const double PQ[3] = {P[0] - tri.C[0], P[1] - tri.C[1], P[2] - tri.C[2]};
+        const double tt = p * g * ipq * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
+        const double pref = sqrt(ipq) * kab * cg;
+        double ur, wr0;
+        rys_root_one<NR>(tt, r, ur, wr0);
+        ur *= ipq;
+        const double qf = g * ur, pf = p * ur;
+        const double b00 = 0.5 * ur, b10 = fma(-hip, qf, hip), b01 = fma(-hg, pf, hg);
+        double gx[LAB1 + 1][LC + 1], gy[LAB1 + 1][LC + 1], gz[LAB1 + 1][LC + 1];
+        rys_vrr<LAB1, LC>(P[0] - tri.A[0] - qf * PQ[0], pf * PQ[0], b10, b01, b00, gx);
+        rys_vrr<LAB1, LC>(P[1] - tri.A[1] - qf * PQ[1], pf * PQ[1], b10, b01, b00, gy);
+        rys_vrr<LAB1, LC>(P[2] - tri.A[2] - qf * PQ[2], pf * PQ[2], b10, b01, b00, gz);
+        const double wr = pref * wr0;
 #pragma unroll
-            for (int z = 0; z < NCC; ++z) {
-              double ix[LA + 2][LB + 2], iy[LA + 2][LB + 2], iz[LA + 2][LB + 2];
-              rys_hrr_col<LA + 1, LB + 1, LC>(gx, cc.x[z], ab[0], ix);
-              rys_hrr_col<LA + 1, LB + 1, LC>(gy, cc.y[z], ab[1], iy);
-              rys_hrr_col<LA + 1, LB + 1, LC>(gz, cc.z[z], ab[2], iz);
+        for (int z = 0; z < NCC; ++z) {
+          double ix[LA + 2][LB + 2], iy[LA + 2][LB + 2], iz[LA + 2][LB + 2];
+          rys_hrr_col<LA + 1, LB + 1, LC>(gx, cc.x[z], tri.ab[0], ix);
+          rys_hrr_col<LA + 1, LB + 1, LC>(gy, cc.y[z], tri.ab[1], iy);
+          rys_hrr_col<LA + 1, LB + 1, LC>(gz, cc.z[z], tri.ab[2], iz);
 #pragma unroll
-              for (int i = 0; i < NCA; ++i)
+          for (int i = 0; i < NCA; ++i)
 #pragma unroll
-                for (int j = 0; j < NCB; ++j) {
-                  const int ax = ca.x[i], ay = ca.y[i], az = ca.z[i];
-                  const int bx = cb.x[j], by = cb.y[j], bz = cb.z[j];
-                  const double x0 = ix[ax][bx], y0 = iy[ay][by], z0 = iz[az][bz];
-                  const double dax = 2.0 * a * ix[ax + 1][bx] - (ax ? ax * ix[ax ? ax - 1 : 0][bx] : 0.0);
-                  const double day = 2.0 * a * iy[ay + 1][by] - (ay ? ay * iy[ay ? ay - 1 : 0][by] : 0.0);
-                  const double daz = 2.0 * a * iz[az + 1][bz] - (az ? az * iz[az ? az - 1 : 0][bz] : 0.0);
-                  const double dbx = 2.0 * b * ix[ax][bx + 1] - (bx ? bx * ix[ax][bx ? bx - 1 : 0] : 0.0);
-                  const double dby = 2.0 * b * iy[ay][by + 1] - (by ? by * iy[ay][by ? by - 1 : 0] : 0.0);
-                  const double dbz = 2.0 * b * iz[az][bz + 1] - (bz ? bz * iz[az][bz ? bz - 1 : 0] : 0.0);
-                  const double ww = wr * wsh[slot][(z * NCA + i) * NCB + j];
-                  gA[0] = fma(ww, dax * y0 * z0, gA[0]);
-                  gA[1] = fma(ww, x0 * day * z0, gA[1]);
-                  gA[2] = fma(ww, x0 * y0 * daz, gA[2]);
-                  gB[0] = fma(ww, dbx * y0 * z0, gB[0]);
-                  gB[1] = fma(ww, x0 * dby * z0, gB[1]);
-                  gB[2] = fma(ww, x0 * y0 * dbz, gB[2]);
-                }
-            }
-          }
+            for (int j = 0; j < NCB; ++j)
+              contract_derivative(ix, iy, iz, ca.x[i], ca.y[i], ca.z[i], cb.x[j], cb.y[j], cb.z[j], a2,
+                                  b2, wr * wsh[slot][(z * NCA + i) * NCB + j], gA, gB);
         }
       }
     }
-  }
+  });
   warp_seg_add(grad, atomA, gA[0], gA[1], gA[2]);
   warp_seg_add(grad, atomB, gB[0], gB[1], gB[2]);
   warp_seg_add(grad, atomC, -(gA[0] + gB[0]), -(gA[1] + gB[1]), -(gA[2] + gB[2]));
@@ -411,7 +382,7 @@ __global__ void __launch_bounds__(round32(Int2cCfg<LA, LC, SPH>::THREADS))
   constexpr int NR = (LA + LC + 1) / 2 + 1;
   constexpr int MODE = SPH ? 0 : 1;
   constexpr Cart<LA> ca{};
-  const ClassMol cm = cms[find_cm_g(cms, ncm, blockIdx.x)];
+  const ClassMol cm = cms[find_cm(cms, ncm, blockIdx.x)];
   const int t0 = (blockIdx.x - cm.chunk_begin) * C::SLOTS;
   const int slot = threadIdx.x / NCC, kc = threadIdx.x % NCC;
   const int t = t0 + slot;
@@ -500,7 +471,7 @@ __global__ void __launch_bounds__(128)
   constexpr int MODE = SPH ? 0 : 1;
   constexpr Cart<LA> ca{};
   constexpr Cart<LB> cb{};
-  const ClassMol cm = cms[find_cm_g(cms, ncm, blockIdx.x)];
+  const ClassMol cm = cms[find_cm(cms, ncm, blockIdx.x)];
   const int t = (blockIdx.x - cm.chunk_begin) * 128 + threadIdx.x;
   if (t >= cm.ntriples) return;
   const DevMol mol = mols[cm.mol];
@@ -654,10 +625,10 @@ template <int LA, int LB, int LC, bool SPH>
 static void glaunch3(const ClassLaunch& cl, const KernelArgs& k, cudaStream_t st) {
   if constexpr (use_root_parallel_g3c(LA, LB, LC)) {
     grad3c_rp_kernel<LA, LB, LC, SPH><<<cl.nblocks, rp_threads_g3c(LA, LB, LC, SPH), 0, st>>>(
-        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, k.w1, k.grad);
+        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, cl.nab, k.w1, k.grad);
   } else {
     grad3c_kernel<LA, LB, LC, SPH><<<cl.nblocks, round32(Int3cCfg<LA, LB, LC, SPH>::THREADS), 0, st>>>(
-        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, k.w1, k.grad);
+        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, cl.nab, k.w1, k.grad);
   }
 }
 

@@ -29,16 +29,6 @@ __device__ __forceinline__ void cart_of(int l, int k, int& x, int& y, int& z) {
   z = rem;
 }
 
-// chunk -> class-molecule entry by binary search over chunk_begin
-__device__ __forceinline__ int find_cm(const ClassMol* __restrict__ cms, int ncm, int block) {
-  int lo = 0, hi = ncm - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (cms[mid].chunk_begin <= block) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
 // transform an (NCA x NCB) Cartesian block with the a/b output transforms
 template <int LA, int LB, int NOA, int NOB>
 __device__ __forceinline__ void transform_ab(int mode, const double (&acc)[ncart(LA)][ncart(LB)],
@@ -69,10 +59,10 @@ __device__ __forceinline__ void transform_ab(int mode, const double (&acc)[ncart
 // ---------------------------------------------------------------------------
 
 template <int LA, int LB, int LC, bool SPH>
-__global__ void __launch_bounds__(Int3cCfg<LA, LB, LC, SPH>::THREADS, min_ctas3c(LA, LB, LC))
+__global__ void __launch_bounds__(round32(Int3cCfg<LA, LB, LC, SPH>::THREADS), min_ctas3c(LA, LB, LC))
     int3c_kernel(DevBasis orb, DevBasis aux, const double* __restrict__ xyz,
                  const DevMol* __restrict__ mols, const int2* __restrict__ pairs,
-                 const ClassMol* __restrict__ cms, int ncm, double* __restrict__ out) {
+                 const ClassMol* __restrict__ cms, int ncm, int stride, double* __restrict__ out) {
   using C = Int3cCfg<LA, LB, LC, SPH>;
   constexpr int NCA = ncart(LA), NCB = ncart(LB), NCC = ncart(LC);
   constexpr int NOA = C::NOA, NOB = C::NOB, NOC = C::NOC;
@@ -80,13 +70,21 @@ __global__ void __launch_bounds__(Int3cCfg<LA, LB, LC, SPH>::THREADS, min_ctas3c
   constexpr int MODE = SPH ? 0 : 1;
   constexpr Cart<LA> ca{};
   constexpr Cart<LB> cb{};
-  __shared__ double stage[C::SLOTS][NCC][NOA * NOB];
+  // the primitive pairs, then the staged blocks
+  union Shared {
+    PairTable tab;
+    double stage[C::SLOTS][NCC][NOA * NOB];
+  };
+  __shared__ __align__(16) Shared sh;
+  auto& stage = sh.stage;
 
   const ClassMol cm = cms[find_cm(cms, ncm, blockIdx.x)];
   const int t0 = (blockIdx.x - cm.chunk_begin) * C::SLOTS;
   const int slot = threadIdx.x / NCC, kc = threadIdx.x % NCC;
   const int t = t0 + slot;
-  const bool valid = t < cm.ntriples;
+  const bool valid = slot < C::SLOTS && t < cm.ntriples;
+  const int q0 = t0 / cm.naux;
+  const int npairs = (min(t0 + C::SLOTS, cm.ntriples) - 1) / cm.naux - q0 + 1;
 
   double acc[NCA][NCB];
 #pragma unroll
@@ -94,59 +92,49 @@ __global__ void __launch_bounds__(Int3cCfg<LA, LB, LC, SPH>::THREADS, min_ctas3c
 #pragma unroll
     for (int j = 0; j < NCB; ++j) acc[i][j] = 0.0;
 
-  if (valid) {
-    const int2 pr = pairs[cm.pair_begin + t / cm.naux];
-    const int sc = cm.aux_begin + t % cm.naux;
-    int kx, ky, kz;
-    cart_of(LC, kc, kx, ky, kz);
-    const double* A = xyz + 3 * orb.atom[pr.x];
-    const double* B = xyz + 3 * orb.atom[pr.y];
-    const double* Cc = xyz + 3 * aux.atom[sc];
-    const double ab[3] = {A[0] - B[0], A[1] - B[1], A[2] - B[2]};
-    const double rab2 = ab[0] * ab[0] + ab[1] * ab[1] + ab[2] * ab[2];
-    const int pa0 = orb.prim_off[pr.x], na = orb.nprim[pr.x];
-    const int pb0 = orb.prim_off[pr.y], nb = orb.nprim[pr.y];
-    const int pc0 = aux.prim_off[sc], nc = aux.nprim[sc];
-    for (int ia = 0; ia < na; ++ia) {
-      const double a = orb.exps[pa0 + ia], ca_ = orb.coefs[pa0 + ia];
-      for (int ib = 0; ib < nb; ++ib) {
-        const double b = orb.exps[pb0 + ib], cb_ = orb.coefs[pb0 + ib];
-        const double p = a + b, ip = 1.0 / p;
-        const double kab = exp(-a * b * ip * rab2) * ca_ * cb_;
-        if (fabs(kab) < kPrimPairCut) continue;
-        const double P[3] = {(a * A[0] + b * B[0]) * ip, (a * A[1] + b * B[1]) * ip,
-                             (a * A[2] + b * B[2]) * ip};
-        for (int ic = 0; ic < nc; ++ic) {
-          const double g = aux.exps[pc0 + ic], cg = aux.coefs[pc0 + ic];
-          const double pq = p + g, ipq = 1.0 / pq;
-          const double PQ[3] = {P[0] - Cc[0], P[1] - Cc[1], P[2] - Cc[2]};
-          const double tt = p * g * ipq * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
-          const double pref = 2.0 * kPi * kPi * sqrt(kPi) * ip / g * sqrt(ipq) * kab * cg;
-          double u[NR], w[NR];
-          rys_roots<NR>(tt, u, w);
+  const int2* cpairs = pairs + cm.pair_begin + q0;
+  const int mine = t / cm.naux - q0;
+  int kx, ky, kz;
+  cart_of(LC, kc, kx, ky, kz);
+  Triple tri;
+  if (valid) tri.load(orb, aux, xyz, cpairs[mine], cm.aux_begin + t % cm.naux);
+  for_prim_pairs(sh.tab, orb, xyz, cpairs, npairs, stride, mine, tri.nab,
+                 [&](const PrimPair* e0, const PrimPair* e1) {
+    for (int ic = 0; ic < tri.nc; ++ic) {
+      const double g = ic ? aux.exps[tri.pc0 + ic] : tri.g0, hg = 0.5 / g;
+      const double cg = 2.0 * hg * (ic ? aux.coefs[tri.pc0 + ic] : tri.c0);
+      for (const PrimPair* e = e0; e < e1; ++e) {
+        const double kab = e->k;
+        if (kab == 0.0) continue;
+        const double p = e->p, hip = e->hip, ipq = 1.0 / (p + g);
+        const double P[3] = {e->x, e->y, e->z};
+        const double PQ[3] = {P[0] - tri.C[0], P[1] - tri.C[1], P[2] - tri.C[2]};
+        const double tt = p * g * ipq * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
+        const double pref = sqrt(ipq) * kab * cg;
+        double u[NR], w[NR];
+        rys_roots<NR>(tt, u, w);
 #pragma unroll
-          for (int r = 0; r < NR; ++r) {
-            const double ur = u[r];
-            const double qf = g * ipq * ur, pf = p * ipq * ur;
-            const double b00 = 0.5 * ipq * ur;
-            const double b10 = 0.5 * ip * (1.0 - qf);
-            const double b01 = 0.5 / g * (1.0 - pf);
-            double ix[LA + 1][LB + 1], iy[LA + 1][LB + 1], iz[LA + 1][LB + 1];
-            rys_2d<LA, LB, LC>(P[0] - A[0] - qf * PQ[0], pf * PQ[0], b10, b01, b00, ab[0], kx, ix);
-            rys_2d<LA, LB, LC>(P[1] - A[1] - qf * PQ[1], pf * PQ[1], b10, b01, b00, ab[1], ky, iy);
-            rys_2d<LA, LB, LC>(P[2] - A[2] - qf * PQ[2], pf * PQ[2], b10, b01, b00, ab[2], kz, iz);
-            const double wr = pref * w[r];
+        for (int r = 0; r < NR; ++r) {
+          const double ur = ipq * u[r];
+          const double qf = g * ur, pf = p * ur;
+          const double b00 = 0.5 * ur;
+          const double b10 = fma(-hip, qf, hip);
+          const double b01 = fma(-hg, pf, hg);
+          double ix[LA + 1][LB + 1], iy[LA + 1][LB + 1], iz[LA + 1][LB + 1];
+          rys_2d<LA, LB, LC>(P[0] - tri.A[0] - qf * PQ[0], pf * PQ[0], b10, b01, b00, tri.ab[0], kx, ix);
+          rys_2d<LA, LB, LC>(P[1] - tri.A[1] - qf * PQ[1], pf * PQ[1], b10, b01, b00, tri.ab[1], ky, iy);
+          rys_2d<LA, LB, LC>(P[2] - tri.A[2] - qf * PQ[2], pf * PQ[2], b10, b01, b00, tri.ab[2], kz, iz);
+          const double wr = pref * w[r];
 #pragma unroll
-            for (int i = 0; i < NCA; ++i)
+          for (int i = 0; i < NCA; ++i)
 #pragma unroll
-              for (int j = 0; j < NCB; ++j)
-                acc[i][j] = fma(wr * ix[ca.x[i]][cb.x[j]],
-                                iy[ca.y[i]][cb.y[j]] * iz[ca.z[i]][cb.z[j]], acc[i][j]);
-          }
+            for (int j = 0; j < NCB; ++j)
+              acc[i][j] = fma(wr * ix[ca.x[i]][cb.x[j]],
+                              iy[ca.y[i]][cb.y[j]] * iz[ca.z[i]][cb.z[j]], acc[i][j]);
         }
       }
     }
-  }
+  });
   double wsph[NOA][NOB];
   transform_ab<LA, LB, NOA, NOB>(MODE, acc, wsph);
   if (threadIdx.x < C::THREADS) {
@@ -160,7 +148,7 @@ __global__ void __launch_bounds__(Int3cCfg<LA, LB, LC, SPH>::THREADS, min_ctas3c
   const DevMol mol = mols[cm.mol];
   constexpr int PER_IJ = C::SLOTS * NOC;
   constexpr int TOTAL = PER_IJ * NOA * NOB;
-  for (int o = threadIdx.x; o < TOTAL; o += C::THREADS) {
+  for (int o = threadIdx.x; o < TOTAL; o += blockDim.x) {
     const int ij = o / PER_IJ, r = o - ij * PER_IJ;
     const int s = r / NOC, k = r - s * NOC;
     const int ts = t0 + s;
@@ -204,10 +192,10 @@ __host__ __device__ constexpr int rp_threads3c(int la, int lb, int lc, bool sph)
 }
 
 template <int LA, int LB, int LC, bool SPH>
-__global__ void __launch_bounds__(rp_threads3c(LA, LB, LC, SPH), min_ctas_rp(rp_threads3c(LA, LB, LC, SPH)))
+__global__ void __launch_bounds__(rp_threads3c(LA, LB, LC, SPH), min_ctas_rp(rp_threads3c(LA, LB, LC, SPH), LA + LB + LC))
     int3c_rp_kernel(DevBasis orb, DevBasis aux, const double* __restrict__ xyz,
                     const DevMol* __restrict__ mols, const int2* __restrict__ pairs,
-                    const ClassMol* __restrict__ cms, int ncm, double* __restrict__ out) {
+                    const ClassMol* __restrict__ cms, int ncm, int stride, double* __restrict__ out) {
   using C = Int3cCfg<LA, LB, LC, SPH>;
   constexpr int NCA = ncart(LA), NCB = ncart(LB), NCC = ncart(LC);
   constexpr int NOA = C::NOA, NOB = C::NOB, NOC = C::NOC;
@@ -217,13 +205,21 @@ __global__ void __launch_bounds__(rp_threads3c(LA, LB, LC, SPH), min_ctas_rp(rp_
   constexpr Cart<LA> ca{};
   constexpr Cart<LB> cb{};
   constexpr Cart<LC> cc{};
-  __shared__ double part[C::SLOTS][NR][NCC][NOA * NOB];
+  // the primitive pairs, then the roots' partial blocks
+  union Shared {
+    PairTable tab;
+    double part[C::SLOTS][NR][NCC][NOA * NOB];
+  };
+  __shared__ __align__(16) Shared sh;
+  auto& part = sh.part;
 
   const ClassMol cm = cms[find_cm(cms, ncm, blockIdx.x)];
   const int t0 = (blockIdx.x - cm.chunk_begin) * C::SLOTS;
   const int slot = threadIdx.x / NR, r = threadIdx.x % NR;
   const int t = t0 + slot;
   const bool valid = slot < C::SLOTS && t < cm.ntriples;
+  const int q0 = t0 / cm.naux;
+  const int npairs = (min(t0 + C::SLOTS, cm.ntriples) - 1) / cm.naux - q0 + 1;
 
   double acc[NCC][NCA][NCB];
 #pragma unroll
@@ -233,60 +229,51 @@ __global__ void __launch_bounds__(rp_threads3c(LA, LB, LC, SPH), min_ctas_rp(rp_
 #pragma unroll
       for (int j = 0; j < NCB; ++j) acc[k][i][j] = 0.0;
 
-  if (valid) {
-    const int2 pr = pairs[cm.pair_begin + t / cm.naux];
-    const int sc = cm.aux_begin + t % cm.naux;
-    const double* A = xyz + 3 * orb.atom[pr.x];
-    const double* B = xyz + 3 * orb.atom[pr.y];
-    const double* Cc = xyz + 3 * aux.atom[sc];
-    const double ab[3] = {A[0] - B[0], A[1] - B[1], A[2] - B[2]};
-    const double rab2 = ab[0] * ab[0] + ab[1] * ab[1] + ab[2] * ab[2];
-    const int pa0 = orb.prim_off[pr.x], na = orb.nprim[pr.x];
-    const int pb0 = orb.prim_off[pr.y], nb = orb.nprim[pr.y];
-    const int pc0 = aux.prim_off[sc], nc = aux.nprim[sc];
-    for (int ia = 0; ia < na; ++ia) {
-      const double a = orb.exps[pa0 + ia], ca_ = orb.coefs[pa0 + ia];
-      for (int ib = 0; ib < nb; ++ib) {
-        const double b = orb.exps[pb0 + ib], cb_ = orb.coefs[pb0 + ib];
-        const double p = a + b, ip = 1.0 / p;
-        const double kab = exp(-a * b * ip * rab2) * ca_ * cb_;
-        if (fabs(kab) < kPrimPairCut) continue;
-        const double P[3] = {(a * A[0] + b * B[0]) * ip, (a * A[1] + b * B[1]) * ip,
-                             (a * A[2] + b * B[2]) * ip};
-        for (int ic = 0; ic < nc; ++ic) {
-          const double g = aux.exps[pc0 + ic], cg = aux.coefs[pc0 + ic];
-          const double pq = p + g, ipq = 1.0 / pq;
-          const double PQ[3] = {P[0] - Cc[0], P[1] - Cc[1], P[2] - Cc[2]};
-          const double tt = p * g * ipq * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
-          const double pref = 2.0 * kPi * kPi * sqrt(kPi) * ip / g * sqrt(ipq) * kab * cg;
-          double ur, wr0;
-          rys_root_one<NR>(tt, r, ur, wr0);
-          const double qf = g * ipq * ur, pf = p * ipq * ur;
-          const double b00 = 0.5 * ipq * ur;
-          const double b10 = 0.5 * ip * (1.0 - qf);
-          const double b01 = 0.5 / g * (1.0 - pf);
-          double gx[LAB + 1][LC + 1], gy[LAB + 1][LC + 1], gz[LAB + 1][LC + 1];
-          rys_vrr<LAB, LC>(P[0] - A[0] - qf * PQ[0], pf * PQ[0], b10, b01, b00, gx);
-          rys_vrr<LAB, LC>(P[1] - A[1] - qf * PQ[1], pf * PQ[1], b10, b01, b00, gy);
-          rys_vrr<LAB, LC>(P[2] - A[2] - qf * PQ[2], pf * PQ[2], b10, b01, b00, gz);
-          const double wr = pref * wr0;
+  const int2* cpairs = pairs + cm.pair_begin + q0;
+  const int mine = t / cm.naux - q0;
+  Triple tri;
+  if (valid) tri.load(orb, aux, xyz, cpairs[mine], cm.aux_begin + t % cm.naux);
+  for_prim_pairs(sh.tab, orb, xyz, cpairs, npairs, stride, mine, tri.nab,
+                 [&](const PrimPair* e0, const PrimPair* e1) {
+    for (int ic = 0; ic < tri.nc; ++ic) {
+      const double g = ic ? aux.exps[tri.pc0 + ic] : tri.g0, hg = 0.5 / g;
+      const double cg = 2.0 * hg * (ic ? aux.coefs[tri.pc0 + ic] : tri.c0);
+      for (const PrimPair* e = e0; e < e1; ++e) {
+        const double kab = e->k;
+        if (kab == 0.0) continue;
+        const double p = e->p, hip = e->hip, ipq = 1.0 / (p + g);
+        const double P[3] = {e->x, e->y, e->z};
+        const double PQ[3] = {P[0] - tri.C[0], P[1] - tri.C[1], P[2] - tri.C[2]};
+        const double tt = p * g * ipq * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
+        const double pref = sqrt(ipq) * kab * cg;
+        double ur, wr0;
+        rys_root_one<NR>(tt, r, ur, wr0);
+        ur *= ipq;
+        const double qf = g * ur, pf = p * ur;
+        const double b00 = 0.5 * ur;
+        const double b10 = fma(-hip, qf, hip);
+        const double b01 = fma(-hg, pf, hg);
+        double gx[LAB + 1][LC + 1], gy[LAB + 1][LC + 1], gz[LAB + 1][LC + 1];
+        rys_vrr<LAB, LC>(P[0] - tri.A[0] - qf * PQ[0], pf * PQ[0], b10, b01, b00, gx);
+        rys_vrr<LAB, LC>(P[1] - tri.A[1] - qf * PQ[1], pf * PQ[1], b10, b01, b00, gy);
+        rys_vrr<LAB, LC>(P[2] - tri.A[2] - qf * PQ[2], pf * PQ[2], b10, b01, b00, gz);
+        const double wr = pref * wr0;
 #pragma unroll
-          for (int k = 0; k < NCC; ++k) {
-            double ix[LA + 1][LB + 1], iy[LA + 1][LB + 1], iz[LA + 1][LB + 1];
-            rys_hrr_col<LA, LB, LC>(gx, cc.x[k], ab[0], ix);
-            rys_hrr_col<LA, LB, LC>(gy, cc.y[k], ab[1], iy);
-            rys_hrr_col<LA, LB, LC>(gz, cc.z[k], ab[2], iz);
+        for (int k = 0; k < NCC; ++k) {
+          double ix[LA + 1][LB + 1], iy[LA + 1][LB + 1], iz[LA + 1][LB + 1];
+          rys_hrr_col<LA, LB, LC>(gx, cc.x[k], tri.ab[0], ix);
+          rys_hrr_col<LA, LB, LC>(gy, cc.y[k], tri.ab[1], iy);
+          rys_hrr_col<LA, LB, LC>(gz, cc.z[k], tri.ab[2], iz);
 #pragma unroll
-            for (int i = 0; i < NCA; ++i)
+          for (int i = 0; i < NCA; ++i)
 #pragma unroll
-              for (int j = 0; j < NCB; ++j)
-                acc[k][i][j] = fma(wr * ix[ca.x[i]][cb.x[j]], iy[ca.y[i]][cb.y[j]] * iz[ca.z[i]][cb.z[j]],
-                                   acc[k][i][j]);
-          }
+            for (int j = 0; j < NCB; ++j)
+              acc[k][i][j] = fma(wr * ix[ca.x[i]][cb.x[j]], iy[ca.y[i]][cb.y[j]] * iz[ca.z[i]][cb.z[j]],
+                                 acc[k][i][j]);
         }
       }
     }
-  }
+  });
   if (slot < C::SLOTS) {
 #pragma unroll
     for (int k = 0; k < NCC; ++k) {
@@ -332,7 +319,7 @@ __global__ void __launch_bounds__(rp_threads3c(LA, LB, LC, SPH), min_ctas_rp(rp_
 // ---------------------------------------------------------------------------
 
 template <int LA, int LC, bool SPH>
-__global__ void __launch_bounds__(Int2cCfg<LA, LC, SPH>::THREADS)
+__global__ void __launch_bounds__(round32(Int2cCfg<LA, LC, SPH>::THREADS))
     int2c_kernel(DevBasis aux, const double* __restrict__ xyz, const DevMol* __restrict__ mols,
                  const int2* __restrict__ pairs, const ClassMol* __restrict__ cms, int ncm,
                  double* __restrict__ out) {
@@ -348,7 +335,7 @@ __global__ void __launch_bounds__(Int2cCfg<LA, LC, SPH>::THREADS)
   const int t0 = (blockIdx.x - cm.chunk_begin) * C::SLOTS;
   const int slot = threadIdx.x / NCC, kc = threadIdx.x % NCC;
   const int t = t0 + slot;
-  const bool valid = t < cm.ntriples;
+  const bool valid = slot < C::SLOTS && t < cm.ntriples;
   double acc[NCA][1];
 #pragma unroll
   for (int i = 0; i < NCA; ++i) acc[i][0] = 0.0;
@@ -396,7 +383,7 @@ __global__ void __launch_bounds__(Int2cCfg<LA, LC, SPH>::THREADS)
   __syncthreads();
   const DevMol mol = mols[cm.mol];
   constexpr int TOTAL = C::SLOTS * NOC * NOA;
-  for (int o = threadIdx.x; o < TOTAL; o += C::THREADS) {
+  for (int o = threadIdx.x; o < TOTAL; o += blockDim.x) {
     const int i = o / (C::SLOTS * NOC), r = o - i * (C::SLOTS * NOC);
     const int s = r / NOC, k = r - s * NOC;
     const int ts = t0 + s;
@@ -554,16 +541,16 @@ template <int LA, int LB, int LC, bool SPH>
 static void launch3(const ClassLaunch& cl, const KernelArgs& k, cudaStream_t st) {
   if constexpr (use_root_parallel3c(LA, LB, LC, SPH)) {
     int3c_rp_kernel<LA, LB, LC, SPH><<<cl.nblocks, rp_threads3c(LA, LB, LC, SPH), 0, st>>>(
-        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, k.out);
+        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, cl.nab, k.out);
   } else {
-    int3c_kernel<LA, LB, LC, SPH><<<cl.nblocks, Int3cCfg<LA, LB, LC, SPH>::THREADS, 0, st>>>(
-        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, k.out);
+    int3c_kernel<LA, LB, LC, SPH><<<cl.nblocks, round32(Int3cCfg<LA, LB, LC, SPH>::THREADS), 0, st>>>(
+        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, cl.nab, k.out);
   }
 }
 
 template <int LA, int LC, bool SPH>
 static void launch2(const ClassLaunch& cl, const KernelArgs& k, cudaStream_t st) {
-  int2c_kernel<LA, LC, SPH><<<cl.nblocks, Int2cCfg<LA, LC, SPH>::THREADS, 0, st>>>(
+  int2c_kernel<LA, LC, SPH><<<cl.nblocks, round32(Int2cCfg<LA, LC, SPH>::THREADS), 0, st>>>(
       k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, k.out);
 }
 

@@ -1,7 +1,7 @@
 // Shared device-side definitions for the DF-RHF kernels (sm_100a).
 //
 // Integrals use Rys quadrature (Rys, Dupuis, King, J. Comput. Chem. 4, 154
-// (1983)): nodes/weights come from the piecewise Chebyshev table generated by
+// (1983)): nodes/weights come from the piecewise polynomial table generated by
 // gen_rys_table.py (80-digit Golub-Welsch on Boys moments) and, for large T,
 // from the Gauss-Hermite limit.  Two-dimensional integrals follow the Rys
 // vertical recurrence in (e0|f0) and the horizontal transfer
@@ -33,6 +33,30 @@ __host__ __device__ constexpr int nsph(int l) { return 2 * l + 1; }
 // sph_table.inc: mode 0 = real spherical (PySCF order), mode 1 = normalised
 // Cartesian components.
 
+// Nodes and weights on [0, T_asym): degree-RYS_DEG polynomials on intervals of
+// width RYS_H.  A warp's threads have different T, so the coefficient loads are
+// a gather and the L1 takes about a cycle per thread and load: the table keeps
+// the (u, w) pairs of a root together and two powers come with one 32-byte
+// load (5 loads a root instead of 20 eight-byte ones).  Powers of x instead of
+// a Chebyshev recurrence: one FMA per coefficient instead of an FMA and an
+// addition.
+__device__ __forceinline__ void rys_poly(const double* __restrict__ c, double x, double& u, double& w) {
+  static_assert(RYS_LAYOUT == 2 && RYS_DEG % 2 == 1, "coefficient layout");
+  double a[2 * (RYS_DEG + 1)];
+#pragma unroll
+  for (int k = 0; k < (RYS_DEG + 1) / 2; ++k)
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(a[4 * k]), "=d"(a[4 * k + 1]), "=d"(a[4 * k + 2]), "=d"(a[4 * k + 3])
+        : "l"(c + 4 * k));
+  u = a[0];
+  w = a[1];
+#pragma unroll
+  for (int k = 1; k <= RYS_DEG; ++k) {
+    u = fma(u, x, a[2 * k]);
+    w = fma(w, x, a[2 * k + 1]);
+  }
+}
+
 template <int N>
 __device__ __forceinline__ void rys_roots(double t, double (&u)[N], double (&w)[N]) {
   static_assert(N >= 1 && N <= RYS_NMAX, "root count outside the table");
@@ -42,21 +66,9 @@ __device__ __forceinline__ void rys_roots(double t, double (&u)[N], double (&w)[
     int i = (int)(t * (1.0 / RYS_H));
     i = i < 0 ? 0 : (i >= kIntervals ? kIntervals - 1 : i);
     const double x = 2.0 * (t - i * RYS_H) * (1.0 / RYS_H) - 1.0;
-    const double x2 = 2.0 * x;
     const double* c = d_rys_table + kOffset + (size_t)i * (2 * N * (RYS_DEG + 1));
 #pragma unroll
-    for (int s = 0; s < 2 * N; ++s) {
-      const double* cs = c + s * (RYS_DEG + 1);
-      double b1 = 0.0, b2 = 0.0;
-#pragma unroll
-      for (int k = RYS_DEG; k > 0; --k) {
-        const double b0 = fma(x2, b1, __ldg(cs + k) - b2);
-        b2 = b1;
-        b1 = b0;
-      }
-      const double v = fma(x, b1, __ldg(cs) - b2);
-      if (s < N) u[s] = v; else w[s - N] = v;
-    }
+    for (int s = 0; s < N; ++s) rys_poly(c + s * (2 * (RYS_DEG + 1)), x, u[s], w[s]);
   } else {
     const double inv = 1.0 / t;
     const double rs = sqrt(inv);
@@ -118,7 +130,7 @@ __device__ __forceinline__ void rys_2d(double c00, double c00p, double b10, doub
 }
 
 // One root of the Rys quadrature (node u_r, weight w_r) for a runtime index
-// r < N: the two Chebyshev series of that root only.
+// r < N.
 template <int N>
 __device__ __forceinline__ void rys_root_one(double t, int r, double& u, double& w) {
   static_assert(N >= 1 && N <= RYS_NMAX, "root count outside the table");
@@ -128,22 +140,7 @@ __device__ __forceinline__ void rys_root_one(double t, int r, double& u, double&
     int i = (int)(t * (1.0 / RYS_H));
     i = i < 0 ? 0 : (i >= kIntervals ? kIntervals - 1 : i);
     const double x = 2.0 * (t - i * RYS_H) * (1.0 / RYS_H) - 1.0;
-    const double x2 = 2.0 * x;
-    const double* c = d_rys_table + kOffset + (size_t)i * (2 * N * (RYS_DEG + 1));
-    const double* cu = c + r * (RYS_DEG + 1);
-    const double* cw = c + (N + r) * (RYS_DEG + 1);
-    double bu1 = 0.0, bu2 = 0.0, bw1 = 0.0, bw2 = 0.0;
-#pragma unroll
-    for (int k = RYS_DEG; k > 0; --k) {
-      const double bu0 = fma(x2, bu1, __ldg(cu + k) - bu2);
-      const double bw0 = fma(x2, bw1, __ldg(cw + k) - bw2);
-      bu2 = bu1;
-      bu1 = bu0;
-      bw2 = bw1;
-      bw1 = bw0;
-    }
-    u = fma(x, bu1, __ldg(cu) - bu2);
-    w = fma(x, bw1, __ldg(cw) - bw2);
+    rys_poly(d_rys_table + kOffset + (size_t)(i * N + r) * (2 * (RYS_DEG + 1)), x, u, w);
   } else {
     const double inv = 1.0 / t;
     u = d_rys_x2[N - 1][r] * inv;
