@@ -32,10 +32,40 @@ __device__ __forceinline__ void cart_of_g(int l, int k, int& x, int& y, int& z) 
   z = rem;
 }
 
-// Add v (3 components) to grad[3*key+d] across a full warp, segmented by runs
-// of equal key in lane order; key < 0 contributes nothing.
-__device__ __forceinline__ void warp_seg_add(double* __restrict__ grad, int key, double vx,
-                                             double vy, double vz) {
+// Gradient sums of one molecule in shared memory.  A 3-centre CTA works
+// through a run of launch chunks and adds to global memory when the molecule
+// changes: one global atomic per atom, direction and run of chunks instead of
+// a few per warp.  Every CTA of a launch is on the same few molecules at a
+// time, so those atomics met on a handful of L2 sectors (12 x (H2O)6: (ss|s)
+// 0.226 -> 0.152 ms, (ps|s) 0.302 -> 0.211, (ps|p) 0.409 -> 0.299).  Molecules
+// of more atoms take the global atomics directly.
+constexpr int kAccAtoms = 128;
+struct AtomSums {
+  double v[3 * kAccAtoms];
+};
+
+// Chunks a CTA works through: up to four, as long as eight CTAs per SM remain.
+// One chunk 3.79, two 3.71, four 3.63, eight 3.69, sixteen 3.63 ms for the
+// derivatives of 12 x (H2O)6; 1 x (H2O)16 4.79, 4.58, 4.56, 4.51, 4.55.
+inline int chunks_per_cta(int nblocks) {
+  const int per = nblocks / (148 * 8);
+  return per < 1 ? 1 : (per < 4 ? per : 4);
+}
+
+__device__ __forceinline__ void flush_sums(AtomSums& acc, const DevMol& mol, double* __restrict__ grad) {
+  __syncthreads();
+  for (int i = threadIdx.x; i < 3 * min(mol.natom, kAccAtoms); i += blockDim.x) {
+    const double v = acc.v[i];
+    if (v != 0.0) atomicAdd(grad + 3 * mol.atom_off + i, v);  // NaN != 0: added
+    acc.v[i] = 0.0;
+  }
+  __syncthreads();
+}
+
+// add(3*key+d, v_d) across a full warp, segmented by runs of equal key in lane
+// order; key < 0 contributes nothing.
+template <class Add>
+__device__ __forceinline__ void warp_seg_add(Add&& add, int key, double vx, double vy, double vz) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int prev = __shfl_up_sync(full, key, 1);
@@ -61,9 +91,9 @@ __device__ __forceinline__ void warp_seg_add(double* __restrict__ grad, int key,
   const int next = __shfl_down_sync(full, key, 1);
   const bool tail = lane == 31 || next != key;
   if (tail && key >= 0) {
-    atomicAdd(grad + 3 * key + 0, v[0]);
-    atomicAdd(grad + 3 * key + 1, v[1]);
-    atomicAdd(grad + 3 * key + 2, v[2]);
+    add(3 * key + 0, v[0]);
+    add(3 * key + 1, v[1]);
+    add(3 * key + 2, v[2]);
   }
 }
 
@@ -126,7 +156,7 @@ __global__ void __launch_bounds__(round32(Int3cCfg<LA, LB, LC, SPH>::THREADS),
                                   min_ctas_grad3c(LA, LB, LC))
     grad3c_kernel(DevBasis orb, DevBasis aux, const double* __restrict__ xyz,
                   const DevMol* __restrict__ mols, const int2* __restrict__ pairs,
-                  const ClassMol* __restrict__ cms, int ncm, int stride, const double* __restrict__ abar,
+                  const ClassMol* __restrict__ cms, int ncm, int nblocks, int per_cta, int stride, const double* __restrict__ abar,
                   double* __restrict__ grad) {
   using C = Int3cCfg<LA, LB, LC, SPH>;
   constexpr int NCA = ncart(LA), NCB = ncart(LB), NCC = ncart(LC);
@@ -136,90 +166,107 @@ __global__ void __launch_bounds__(round32(Int3cCfg<LA, LB, LC, SPH>::THREADS),
   constexpr Cart<LA> ca{};
   constexpr Cart<LB> cb{};
 
-  const ClassMol cm = cms[find_cm(cms, ncm, blockIdx.x)];
-  const int t0 = (blockIdx.x - cm.chunk_begin) * C::SLOTS;
-  const int slot = threadIdx.x / NCC, kc = threadIdx.x % NCC;
-  const int t = t0 + slot;
-  const bool valid = slot < C::SLOTS && t < cm.ntriples;
-  const int q0 = t0 / cm.naux;
-  const int npairs = (min(t0 + C::SLOTS, cm.ntriples) - 1) / cm.naux - q0 + 1;
-  const int2* cpairs = pairs + cm.pair_begin + q0;
   __shared__ __align__(16) PairTable tab;
-  double gA[3] = {0.0, 0.0, 0.0}, gB[3] = {0.0, 0.0, 0.0};
-  int atomA = -1, atomB = -1, atomC = -1;
-  int2 pr = make_int2(0, 0);
-  int sc = 0, kx = 0, ky = 0, kz = 0;
-  bool work = false;
-  double wc[NCA][NCB] = {};
-  if (valid) {
-    pr = cpairs[t / cm.naux - q0];
-    sc = cm.aux_begin + t % cm.naux;
-    atomA = orb.atom[pr.x];
-    atomB = orb.atom[pr.y];
-    atomC = aux.atom[sc];
-    work = !(atomA == atomB && atomB == atomC);
-  }
-  Triple tri;
-  if (work) tri.load(orb, aux, xyz, pr, sc);
-  if (work) {
-    const DevMol mol = mols[cm.mol];
-    cart_of_g(LC, kc, kx, ky, kz);
-    // weights: Abar block for this Cartesian aux component, in Cartesian a, b
-    double wsph[NOA][NOB];
-    const int fa = orb.func_off[pr.x], fb = orb.func_off[pr.y], fc = aux.func_off[sc];
+  __shared__ AtomSums sums;
+  for (int i = threadIdx.x; i < 3 * kAccAtoms; i += blockDim.x) sums.v[i] = 0.0;
+  int held = -1, first = 0;  // molecule the sums belong to, its first atom
+  bool local = false;
+  auto add = [&](int i, double v) {
+    if (local) atomicAdd(&sums.v[i - 3 * first], v);
+    else atomicAdd(grad + i, v);
+  };
+  for (int block = blockIdx.x * per_cta; block < min(nblocks, ((int)blockIdx.x + 1) * per_cta); ++block) {
+    const ClassMol cm = cms[find_cm(cms, ncm, block)];
+    if (cm.mol != held) {
+      if (local) flush_sums(sums, mols[held], grad);
+      held = cm.mol;
+      first = mols[held].atom_off;
+      local = mols[held].natom <= kAccAtoms;
+    }
+    const int t0 = (block - cm.chunk_begin) * C::SLOTS;
+    const int slot = threadIdx.x / NCC, kc = threadIdx.x % NCC;
+    const int t = t0 + slot;
+    const bool valid = slot < C::SLOTS && t < cm.ntriples;
+    const int q0 = t0 / cm.naux;
+    const int npairs = (min(t0 + C::SLOTS, cm.ntriples) - 1) / cm.naux - q0 + 1;
+    const int2* cpairs = pairs + cm.pair_begin + q0;
+    double gA[3] = {0.0, 0.0, 0.0}, gB[3] = {0.0, 0.0, 0.0};
+    int atomA = -1, atomB = -1, atomC = -1;
+    int2 pr = make_int2(0, 0);
+    int sc = 0, kx = 0, ky = 0, kz = 0;
+    bool work = false;
+    double wc[NCA][NCB] = {};
+    if (valid) {
+      pr = cpairs[t / cm.naux - q0];
+      sc = cm.aux_begin + t % cm.naux;
+      atomA = orb.atom[pr.x];
+      atomB = orb.atom[pr.y];
+      atomC = aux.atom[sc];
+      work = !(atomA == atomB && atomB == atomC);
+    }
+    Triple tri;
+    if (work) tri.load(orb, aux, xyz, pr, sc);
+    if (work) {
+      const DevMol mol = mols[cm.mol];
+      cart_of_g(LC, kc, kx, ky, kz);
+      // weights: Abar block for this Cartesian aux component, in Cartesian a, b
+      double wsph[NOA][NOB];
+      const int fa = orb.func_off[pr.x], fb = orb.func_off[pr.y], fc = aux.func_off[sc];
 #pragma unroll
-    for (int i = 0; i < NOA; ++i)
+      for (int i = 0; i < NOA; ++i)
 #pragma unroll
-      for (int j = 0; j < NOB; ++j) {
-        const long long mu = fa + i, nu = fb + j;
-        const long long hi = mu > nu ? mu : nu, lo = mu > nu ? nu : mu;
-        const double* row = abar + mol.a_off + (hi * (hi + 1) / 2 + lo) * mol.naux + fc;
-        double s = 0.0;
+        for (int j = 0; j < NOB; ++j) {
+          const long long mu = fa + i, nu = fb + j;
+          const long long hi = mu > nu ? mu : nu, lo = mu > nu ? nu : mu;
+          const double* row = abar + mol.a_off + (hi * (hi + 1) / 2 + lo) * mol.naux + fc;
+          double s = 0.0;
 #pragma unroll
-        for (int k = 0; k < NOC; ++k) s = fma(c_trans[MODE][LC][k][kc], __ldg(row + k), s);
-        wsph[i][j] = s;
-      }
-    weights_to_cart<LA, LB, NOA, NOB>(MODE, wsph, wc);
-  }
-  for_prim_pairs(tab, orb, xyz, cpairs, npairs, stride, t / cm.naux - q0, tri.nab,
-                 [&](const PrimPair* e0, const PrimPair* e1) {
-    const double pair_factor = (pr.x == pr.y) ? 1.0 : 2.0;
-    for (int ic = 0; ic < tri.nc; ++ic) {
-      const double g = ic ? aux.exps[tri.pc0 + ic] : tri.g0, hg = 0.5 / g;
-      const double cg = 2.0 * hg * (ic ? aux.coefs[tri.pc0 + ic] : tri.c0) * pair_factor;
-      for (const PrimPair* e = e0; e < e1; ++e) {
-        const double kab = e->k;
-        if (kab == 0.0) continue;
-        const double p = e->p, hip = e->hip, ipq = 1.0 / (p + g), a2 = e->a2, b2 = e->b2;
-        const double P[3] = {e->x, e->y, e->z};
-        const double PQ[3] = {P[0] - tri.C[0], P[1] - tri.C[1], P[2] - tri.C[2]};
-        const double tt = p * g * ipq * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
-        const double pref = sqrt(ipq) * kab * cg;
-        double u[NR], w[NR];
-        rys_roots<NR>(tt, u, w);
+          for (int k = 0; k < NOC; ++k) s = fma(c_trans[MODE][LC][k][kc], __ldg(row + k), s);
+          wsph[i][j] = s;
+        }
+      weights_to_cart<LA, LB, NOA, NOB>(MODE, wsph, wc);
+    }
+    for_prim_pairs(tab, orb, xyz, cpairs, npairs, stride, t / cm.naux - q0, tri.nab,
+                   [&](const PrimPair* e0, const PrimPair* e1) {
+      const double pair_factor = (pr.x == pr.y) ? 1.0 : 2.0;
+      for (int ic = 0; ic < tri.nc; ++ic) {
+        const double g = ic ? aux.exps[tri.pc0 + ic] : tri.g0, hg = 0.5 / g;
+        const double cg = 2.0 * hg * (ic ? aux.coefs[tri.pc0 + ic] : tri.c0) * pair_factor;
+        for (const PrimPair* e = e0; e < e1; ++e) {
+          const double kab = e->k;
+          if (kab == 0.0) continue;
+          const double p = e->p, hip = e->hip, ipq = 1.0 / (p + g), a2 = e->a2, b2 = e->b2;
+          const double P[3] = {e->x, e->y, e->z};
+          const double PQ[3] = {P[0] - tri.C[0], P[1] - tri.C[1], P[2] - tri.C[2]};
+          const double tt = p * g * ipq * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
+          const double pref = sqrt(ipq) * kab * cg;
+          double u[NR], w[NR];
+          rys_roots<NR>(tt, u, w);
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-          const double ur = ipq * u[r];
-          const double qf = g * ur, pf = p * ur;
-          const double b00 = 0.5 * ur, b10 = fma(-hip, qf, hip), b01 = fma(-hg, pf, hg);
-          double ix[LA + 2][LB + 2], iy[LA + 2][LB + 2], iz[LA + 2][LB + 2];
-          rys_2d<LA + 1, LB + 1, LC>(P[0] - tri.A[0] - qf * PQ[0], pf * PQ[0], b10, b01, b00, tri.ab[0], kx, ix);
-          rys_2d<LA + 1, LB + 1, LC>(P[1] - tri.A[1] - qf * PQ[1], pf * PQ[1], b10, b01, b00, tri.ab[1], ky, iy);
-          rys_2d<LA + 1, LB + 1, LC>(P[2] - tri.A[2] - qf * PQ[2], pf * PQ[2], b10, b01, b00, tri.ab[2], kz, iz);
-          const double wr = pref * w[r];
+          for (int r = 0; r < NR; ++r) {
+            const double ur = ipq * u[r];
+            const double qf = g * ur, pf = p * ur;
+            const double b00 = 0.5 * ur, b10 = fma(-hip, qf, hip), b01 = fma(-hg, pf, hg);
+            double ix[LA + 2][LB + 2], iy[LA + 2][LB + 2], iz[LA + 2][LB + 2];
+            rys_2d<LA + 1, LB + 1, LC>(P[0] - tri.A[0] - qf * PQ[0], pf * PQ[0], b10, b01, b00, tri.ab[0], kx, ix);
+            rys_2d<LA + 1, LB + 1, LC>(P[1] - tri.A[1] - qf * PQ[1], pf * PQ[1], b10, b01, b00, tri.ab[1], ky, iy);
+            rys_2d<LA + 1, LB + 1, LC>(P[2] - tri.A[2] - qf * PQ[2], pf * PQ[2], b10, b01, b00, tri.ab[2], kz, iz);
+            const double wr = pref * w[r];
 #pragma unroll
-          for (int i = 0; i < NCA; ++i)
+            for (int i = 0; i < NCA; ++i)
 #pragma unroll
-            for (int j = 0; j < NCB; ++j)
-              contract_derivative(ix, iy, iz, ca.x[i], ca.y[i], ca.z[i], cb.x[j], cb.y[j], cb.z[j], a2,
-                                  b2, wr * wc[i][j], gA, gB);
+              for (int j = 0; j < NCB; ++j)
+                contract_derivative(ix, iy, iz, ca.x[i], ca.y[i], ca.z[i], cb.x[j], cb.y[j], cb.z[j], a2,
+                                    b2, wr * wc[i][j], gA, gB);
+          }
         }
       }
-    }
-  });
-  warp_seg_add(grad, atomA, gA[0], gA[1], gA[2]);
-  warp_seg_add(grad, atomB, gB[0], gB[1], gB[2]);
-  warp_seg_add(grad, atomC, -(gA[0] + gB[0]), -(gA[1] + gB[1]), -(gA[2] + gB[2]));
+    });
+    warp_seg_add(add, atomA, gA[0], gA[1], gA[2]);
+    warp_seg_add(add, atomB, gB[0], gB[1], gB[2]);
+    warp_seg_add(add, atomC, -(gA[0] + gB[0]), -(gA[1] + gB[1]), -(gA[2] + gB[2]));
+  }
+  if (local) flush_sums(sums, mols[held], grad);
 }
 
 // ---------------------------------------------------------------------------
@@ -246,7 +293,7 @@ __global__ void __launch_bounds__(rp_threads_g3c(LA, LB, LC, SPH),
                                   min_ctas_rp(rp_threads_g3c(LA, LB, LC, SPH), LA + LB + LC))
     grad3c_rp_kernel(DevBasis orb, DevBasis aux, const double* __restrict__ xyz,
                      const DevMol* __restrict__ mols, const int2* __restrict__ pairs,
-                     const ClassMol* __restrict__ cms, int ncm, int stride, const double* __restrict__ abar,
+                     const ClassMol* __restrict__ cms, int ncm, int nblocks, int per_cta, int stride, const double* __restrict__ abar,
                      double* __restrict__ grad) {
   using C = Int3cCfg<LA, LB, LC, SPH>;
   constexpr int NCA = ncart(LA), NCB = ncart(LB), NCC = ncart(LC);
@@ -258,113 +305,130 @@ __global__ void __launch_bounds__(rp_threads_g3c(LA, LB, LC, SPH),
   constexpr Cart<LB> cb{};
   constexpr Cart<LC> cc{};
 
-  const ClassMol cm = cms[find_cm(cms, ncm, blockIdx.x)];
-  const int t0 = (blockIdx.x - cm.chunk_begin) * C::SLOTS;
-  const int slot = threadIdx.x / NR, r = threadIdx.x % NR;
-  const int t = t0 + slot;
-  const bool valid = slot < C::SLOTS && t < cm.ntriples;
-  const int q0 = t0 / cm.naux;
-  const int npairs = (min(t0 + C::SLOTS, cm.ntriples) - 1) / cm.naux - q0 + 1;
-  const int2* cpairs = pairs + cm.pair_begin + q0;
   __shared__ __align__(16) PairTable tab;
-  // contraction weights of every Cartesian aux component, Cartesian in a and
-  // b: one copy per slot in shared memory, formed by the slot's first root
-  // thread and read by all of its roots (a register copy per root thread held
-  // these kernels at 126-255 registers)
-  __shared__ double wsh[C::SLOTS][NCC * NCA * NCB];
-  double gA[3] = {0.0, 0.0, 0.0}, gB[3] = {0.0, 0.0, 0.0};
-  int atomA = -1, atomB = -1, atomC = -1;
-  int2 pr = make_int2(0, 0);
-  int sc = 0;
-  bool work = false;
-  if (valid) {
-    pr = cpairs[t / cm.naux - q0];
-    sc = cm.aux_begin + t % cm.naux;
-    atomA = orb.atom[pr.x];
-    atomB = orb.atom[pr.y];
-    atomC = aux.atom[sc];
-    work = !(atomA == atomB && atomB == atomC);
-  }
-  Triple tri;
-  if (work) tri.load(orb, aux, xyz, pr, sc);
-  if (work && r == 0) {
-    const DevMol mol = mols[cm.mol];
-    const int fa = orb.func_off[pr.x], fb = orb.func_off[pr.y], fc = aux.func_off[sc];
-    double wk[NOA][NOB][NOC];
-#pragma unroll
-    for (int i = 0; i < NOA; ++i)
-#pragma unroll
-      for (int j = 0; j < NOB; ++j) {
-        const long long mu = fa + i, nu = fb + j;
-        const long long hi = mu > nu ? mu : nu, lo = mu > nu ? nu : mu;
-        const double* row = abar + mol.a_off + (hi * (hi + 1) / 2 + lo) * mol.naux + fc;
-#pragma unroll
-        for (int k = 0; k < NOC; ++k) wk[i][j][k] = __ldg(row + k);
-      }
-#pragma unroll
-    for (int z = 0; z < NCC; ++z) {
-      double wsph[NOA][NOB];
+  __shared__ AtomSums sums;
+  for (int i = threadIdx.x; i < 3 * kAccAtoms; i += blockDim.x) sums.v[i] = 0.0;
+  int held = -1, first = 0;  // molecule the sums belong to, its first atom
+  bool local = false;
+  auto add = [&](int i, double v) {
+    if (local) atomicAdd(&sums.v[i - 3 * first], v);
+    else atomicAdd(grad + i, v);
+  };
+  for (int block = blockIdx.x * per_cta; block < min(nblocks, ((int)blockIdx.x + 1) * per_cta); ++block) {
+    const ClassMol cm = cms[find_cm(cms, ncm, block)];
+    if (cm.mol != held) {
+      if (local) flush_sums(sums, mols[held], grad);
+      held = cm.mol;
+      first = mols[held].atom_off;
+      local = mols[held].natom <= kAccAtoms;
+    }
+    const int t0 = (block - cm.chunk_begin) * C::SLOTS;
+    const int slot = threadIdx.x / NR, r = threadIdx.x % NR;
+    const int t = t0 + slot;
+    const bool valid = slot < C::SLOTS && t < cm.ntriples;
+    const int q0 = t0 / cm.naux;
+    const int npairs = (min(t0 + C::SLOTS, cm.ntriples) - 1) / cm.naux - q0 + 1;
+    const int2* cpairs = pairs + cm.pair_begin + q0;
+    // contraction weights of every Cartesian aux component, Cartesian in a and
+    // b: one copy per slot in shared memory, formed by the slot's first root
+    // thread and read by all of its roots (a register copy per root thread held
+    // these kernels at 126-255 registers)
+    __shared__ double wsh[C::SLOTS][NCC * NCA * NCB];
+    double gA[3] = {0.0, 0.0, 0.0}, gB[3] = {0.0, 0.0, 0.0};
+    int atomA = -1, atomB = -1, atomC = -1;
+    int2 pr = make_int2(0, 0);
+    int sc = 0;
+    bool work = false;
+    if (valid) {
+      pr = cpairs[t / cm.naux - q0];
+      sc = cm.aux_begin + t % cm.naux;
+      atomA = orb.atom[pr.x];
+      atomB = orb.atom[pr.y];
+      atomC = aux.atom[sc];
+      work = !(atomA == atomB && atomB == atomC);
+    }
+    Triple tri;
+    if (work) tri.load(orb, aux, xyz, pr, sc);
+    if (work && r == 0) {
+      const DevMol mol = mols[cm.mol];
+      const int fa = orb.func_off[pr.x], fb = orb.func_off[pr.y], fc = aux.func_off[sc];
+      double wk[NOA][NOB][NOC];
 #pragma unroll
       for (int i = 0; i < NOA; ++i)
 #pragma unroll
         for (int j = 0; j < NOB; ++j) {
-          double s = 0.0;
+          const long long mu = fa + i, nu = fb + j;
+          const long long hi = mu > nu ? mu : nu, lo = mu > nu ? nu : mu;
+          const double* row = abar + mol.a_off + (hi * (hi + 1) / 2 + lo) * mol.naux + fc;
 #pragma unroll
-          for (int k = 0; k < NOC; ++k) s = fma(c_trans[MODE][LC][k][z], wk[i][j][k], s);
-          wsph[i][j] = s;
+          for (int k = 0; k < NOC; ++k) wk[i][j][k] = __ldg(row + k);
         }
-      double wcz[NCA][NCB];
-      weights_to_cart<LA, LB, NOA, NOB>(MODE, wsph, wcz);
 #pragma unroll
-      for (int i = 0; i < NCA; ++i)
+      for (int z = 0; z < NCC; ++z) {
+        double wsph[NOA][NOB];
 #pragma unroll
-        for (int j = 0; j < NCB; ++j) wsh[slot][(z * NCA + i) * NCB + j] = wcz[i][j];
-    }
-  }
-  // (for_prim_pairs synchronises the CTA before any thread reads the weights)
-  for_prim_pairs(tab, orb, xyz, cpairs, npairs, stride, t / cm.naux - q0, tri.nab,
-                 [&](const PrimPair* e0, const PrimPair* e1) {
-    const double pair_factor = (pr.x == pr.y) ? 1.0 : 2.0;
-    for (int ic = 0; ic < tri.nc; ++ic) {
-      const double g = ic ? aux.exps[tri.pc0 + ic] : tri.g0, hg = 0.5 / g;
-      const double cg = 2.0 * hg * (ic ? aux.coefs[tri.pc0 + ic] : tri.c0) * pair_factor;
-      for (const PrimPair* e = e0; e < e1; ++e) {
-        const double kab = e->k;
-        if (kab == 0.0) continue;
-        const double p = e->p, hip = e->hip, ipq = 1.0 / (p + g), a2 = e->a2, b2 = e->b2;
-        const double P[3] = {e->x, e->y, e->z};
-        const double PQ[3] = {P[0] - tri.C[0], P[1] - tri.C[1], P[2] - tri.C[2]};
-        const double tt = p * g * ipq * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
-        const double pref = sqrt(ipq) * kab * cg;
-        double ur, wr0;
-        rys_root_one<NR>(tt, r, ur, wr0);
-        ur *= ipq;
-        const double qf = g * ur, pf = p * ur;
-        const double b00 = 0.5 * ur, b10 = fma(-hip, qf, hip), b01 = fma(-hg, pf, hg);
-        double gx[LAB1 + 1][LC + 1], gy[LAB1 + 1][LC + 1], gz[LAB1 + 1][LC + 1];
-        rys_vrr<LAB1, LC>(P[0] - tri.A[0] - qf * PQ[0], pf * PQ[0], b10, b01, b00, gx);
-        rys_vrr<LAB1, LC>(P[1] - tri.A[1] - qf * PQ[1], pf * PQ[1], b10, b01, b00, gy);
-        rys_vrr<LAB1, LC>(P[2] - tri.A[2] - qf * PQ[2], pf * PQ[2], b10, b01, b00, gz);
-        const double wr = pref * wr0;
+        for (int i = 0; i < NOA; ++i)
 #pragma unroll
-        for (int z = 0; z < NCC; ++z) {
-          double ix[LA + 2][LB + 2], iy[LA + 2][LB + 2], iz[LA + 2][LB + 2];
-          rys_hrr_col<LA + 1, LB + 1, LC>(gx, cc.x[z], tri.ab[0], ix);
-          rys_hrr_col<LA + 1, LB + 1, LC>(gy, cc.y[z], tri.ab[1], iy);
-          rys_hrr_col<LA + 1, LB + 1, LC>(gz, cc.z[z], tri.ab[2], iz);
+          for (int j = 0; j < NOB; ++j) {
+            double s = 0.0;
 #pragma unroll
-          for (int i = 0; i < NCA; ++i)
+            for (int k = 0; k < NOC; ++k) s = fma(c_trans[MODE][LC][k][z], wk[i][j][k], s);
+            wsph[i][j] = s;
+          }
+        double wcz[NCA][NCB];
+        weights_to_cart<LA, LB, NOA, NOB>(MODE, wsph, wcz);
 #pragma unroll
-            for (int j = 0; j < NCB; ++j)
-              contract_derivative(ix, iy, iz, ca.x[i], ca.y[i], ca.z[i], cb.x[j], cb.y[j], cb.z[j], a2,
-                                  b2, wr * wsh[slot][(z * NCA + i) * NCB + j], gA, gB);
-        }
+        for (int i = 0; i < NCA; ++i)
+#pragma unroll
+          for (int j = 0; j < NCB; ++j) wsh[slot][(z * NCA + i) * NCB + j] = wcz[i][j];
       }
     }
-  });
-  warp_seg_add(grad, atomA, gA[0], gA[1], gA[2]);
-  warp_seg_add(grad, atomB, gB[0], gB[1], gB[2]);
-  warp_seg_add(grad, atomC, -(gA[0] + gB[0]), -(gA[1] + gB[1]), -(gA[2] + gB[2]));
+    // (for_prim_pairs synchronises the CTA before any thread reads the weights)
+    for_prim_pairs(tab, orb, xyz, cpairs, npairs, stride, t / cm.naux - q0, tri.nab,
+                   [&](const PrimPair* e0, const PrimPair* e1) {
+      const double pair_factor = (pr.x == pr.y) ? 1.0 : 2.0;
+      for (int ic = 0; ic < tri.nc; ++ic) {
+        const double g = ic ? aux.exps[tri.pc0 + ic] : tri.g0, hg = 0.5 / g;
+        const double cg = 2.0 * hg * (ic ? aux.coefs[tri.pc0 + ic] : tri.c0) * pair_factor;
+        for (const PrimPair* e = e0; e < e1; ++e) {
+          const double kab = e->k;
+          if (kab == 0.0) continue;
+          const double p = e->p, hip = e->hip, ipq = 1.0 / (p + g), a2 = e->a2, b2 = e->b2;
+          const double P[3] = {e->x, e->y, e->z};
+          const double PQ[3] = {P[0] - tri.C[0], P[1] - tri.C[1], P[2] - tri.C[2]};
+          const double tt = p * g * ipq * (PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2]);
+          const double pref = sqrt(ipq) * kab * cg;
+          double ur, wr0;
+          rys_root_one<NR>(tt, r, ur, wr0);
+          ur *= ipq;
+          const double qf = g * ur, pf = p * ur;
+          const double b00 = 0.5 * ur, b10 = fma(-hip, qf, hip), b01 = fma(-hg, pf, hg);
+          double gx[LAB1 + 1][LC + 1], gy[LAB1 + 1][LC + 1], gz[LAB1 + 1][LC + 1];
+          rys_vrr<LAB1, LC>(P[0] - tri.A[0] - qf * PQ[0], pf * PQ[0], b10, b01, b00, gx);
+          rys_vrr<LAB1, LC>(P[1] - tri.A[1] - qf * PQ[1], pf * PQ[1], b10, b01, b00, gy);
+          rys_vrr<LAB1, LC>(P[2] - tri.A[2] - qf * PQ[2], pf * PQ[2], b10, b01, b00, gz);
+          const double wr = pref * wr0;
+#pragma unroll
+          for (int z = 0; z < NCC; ++z) {
+            double ix[LA + 2][LB + 2], iy[LA + 2][LB + 2], iz[LA + 2][LB + 2];
+            rys_hrr_col<LA + 1, LB + 1, LC>(gx, cc.x[z], tri.ab[0], ix);
+            rys_hrr_col<LA + 1, LB + 1, LC>(gy, cc.y[z], tri.ab[1], iy);
+            rys_hrr_col<LA + 1, LB + 1, LC>(gz, cc.z[z], tri.ab[2], iz);
+#pragma unroll
+            for (int i = 0; i < NCA; ++i)
+#pragma unroll
+              for (int j = 0; j < NCB; ++j)
+                contract_derivative(ix, iy, iz, ca.x[i], ca.y[i], ca.z[i], cb.x[j], cb.y[j], cb.z[j], a2,
+                                    b2, wr * wsh[slot][(z * NCA + i) * NCB + j], gA, gB);
+          }
+        }
+      }
+    });
+    warp_seg_add(add, atomA, gA[0], gA[1], gA[2]);
+    warp_seg_add(add, atomB, gB[0], gB[1], gB[2]);
+    warp_seg_add(add, atomC, -(gA[0] + gB[0]), -(gA[1] + gB[1]), -(gA[2] + gB[2]));
+  }
+  if (local) flush_sums(sums, mols[held], grad);
 }
 
 // ---------------------------------------------------------------------------
@@ -451,8 +515,9 @@ __global__ void __launch_bounds__(round32(Int2cCfg<LA, LC, SPH>::THREADS))
       if (pr.x == pr.y) gA[0] = gA[1] = gA[2] = 0.0;  // unreachable: same atom
     }
   }
-  warp_seg_add(grad, atomA, gA[0], gA[1], gA[2]);
-  warp_seg_add(grad, atomC, -gA[0], -gA[1], -gA[2]);
+  auto add = [&](int i, double v) { atomicAdd(grad + i, v); };
+  warp_seg_add(add, atomA, gA[0], gA[1], gA[2]);
+  warp_seg_add(add, atomC, -gA[0], -gA[1], -gA[2]);
 }
 
 // ---------------------------------------------------------------------------
@@ -623,12 +688,13 @@ __global__ void __launch_bounds__(128)
 
 template <int LA, int LB, int LC, bool SPH>
 static void glaunch3(const ClassLaunch& cl, const KernelArgs& k, cudaStream_t st) {
+  const int per = chunks_per_cta(cl.nblocks), grid = (cl.nblocks + per - 1) / per;
   if constexpr (use_root_parallel_g3c(LA, LB, LC)) {
-    grad3c_rp_kernel<LA, LB, LC, SPH><<<cl.nblocks, rp_threads_g3c(LA, LB, LC, SPH), 0, st>>>(
-        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, cl.nab, k.w1, k.grad);
+    grad3c_rp_kernel<LA, LB, LC, SPH><<<grid, rp_threads_g3c(LA, LB, LC, SPH), 0, st>>>(
+        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, cl.nblocks, per, cl.nab, k.w1, k.grad);
   } else {
-    grad3c_kernel<LA, LB, LC, SPH><<<cl.nblocks, round32(Int3cCfg<LA, LB, LC, SPH>::THREADS), 0, st>>>(
-        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, cl.nab, k.w1, k.grad);
+    grad3c_kernel<LA, LB, LC, SPH><<<grid, round32(Int3cCfg<LA, LB, LC, SPH>::THREADS), 0, st>>>(
+        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, cl.nblocks, per, cl.nab, k.w1, k.grad);
   }
 }
 
