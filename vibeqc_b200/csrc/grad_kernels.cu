@@ -524,6 +524,8 @@ __global__ void __launch_bounds__(round32(Int2cCfg<LA, LC, SPH>::THREADS))
 // one-electron derivative contraction: D d(T + V) - W dS
 // ---------------------------------------------------------------------------
 
+// k1eLanes lanes per shell pair (Lanes1e), nuclei before primitive pairs: one
+// sum per pair and nucleus leaves the registers
 template <int LA, int LB, bool SPH>
 __global__ void __launch_bounds__(128)
     grad1e_kernel(DevBasis orb, const double* __restrict__ xyz, const double* __restrict__ charge,
@@ -536,11 +538,22 @@ __global__ void __launch_bounds__(128)
   constexpr int MODE = SPH ? 0 : 1;
   constexpr Cart<LA> ca{};
   constexpr Cart<LB> cb{};
-  const ClassMol cm = cms[find_cm(cms, ncm, blockIdx.x)];
-  const int t = (blockIdx.x - cm.chunk_begin) * 128 + threadIdx.x;
-  if (t >= cm.ntriples) return;
+  __shared__ AtomSums sums;
+  for (int i = threadIdx.x; i < 3 * kAccAtoms; i += blockDim.x) sums.v[i] = 0.0;
+  __syncthreads();
+  const int chunk = blockIdx.x / k1eLanes;
+  const ClassMol cm = cms[find_cm(cms, ncm, chunk)];
+  const int t = (chunk - cm.chunk_begin) * 128 +
+                ((blockIdx.x % k1eLanes) * 128 + threadIdx.x) / k1eLanes;
+  const bool valid = t < cm.ntriples;
   const DevMol mol = mols[cm.mol];
-  const int2 pr = pairs[cm.pair_begin + t];
+  const bool local = mol.natom <= kAccAtoms;
+  auto add = [&](int i, double v) {
+    if (local) atomicAdd(&sums.v[i - 3 * mol.atom_off], v);
+    else atomicAdd(grad + i, v);
+  };
+  const Lanes1e ln(mol.natom);
+  const int2 pr = pairs[cm.pair_begin + (valid ? t : 0)];
   const int atomA = orb.atom[pr.x], atomB = orb.atom[pr.y];
   const double factor = (pr.x == pr.y) ? 1.0 : 2.0;
   double dw[NOA][NOB], ww[NOA][NOB];
@@ -559,127 +572,143 @@ __global__ void __launch_bounds__(128)
   const double* B = xyz + 3 * atomB;
   const double ab[3] = {A[0] - B[0], A[1] - B[1], A[2] - B[2]};
   const double rab2 = ab[0] * ab[0] + ab[1] * ab[1] + ab[2] * ab[2];
-  const int pa0 = orb.prim_off[pr.x], na = orb.nprim[pr.x];
+  const int pa0 = orb.prim_off[pr.x];
   const int pb0 = orb.prim_off[pr.y], nb = orb.nprim[pr.y];
+  const int nab = valid ? orb.nprim[pr.x] * nb : 0;
   double gst[3] = {0.0, 0.0, 0.0};  // d/dA of (D T - W S); B gets the negative
   double gvA[3] = {0.0, 0.0, 0.0}, gvB[3] = {0.0, 0.0, 0.0};
-  for (int ia = 0; ia < na; ++ia) {
-    const double a = orb.exps[pa0 + ia], ca_ = orb.coefs[pa0 + ia];
-    for (int ib = 0; ib < nb; ++ib) {
-      const double b = orb.exps[pb0 + ib], cb_ = orb.coefs[pb0 + ib];
+  if (atomA != atomB)
+    for (int k = ln.lane; k < nab; k += k1eLanes) {
+      const int ia = pa0 + k / nb, ib = pb0 + k % nb;
+      const double a = orb.exps[ia], b = orb.exps[ib];
       const double p = a + b, ip = 1.0 / p;
-      const double kab = exp(-a * b * ip * rab2) * ca_ * cb_;
+      const double kab = exp(-a * b * ip * rab2) * orb.coefs[ia] * orb.coefs[ib];
       const double P[3] = {(a * A[0] + b * B[0]) * ip, (a * A[1] + b * B[1]) * ip,
                            (a * A[2] + b * B[2]) * ip};
-      if (atomA != atomB) {
-        double s1[3][LA + 2][LB + 3], t1[3][LA + 2][LB + 1];
+      double s1[3][LA + 2][LB + 3], t1[3][LA + 2][LB + 1];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          const double xpa = P[d] - A[d], xpb = P[d] - B[d];
-          double s[LA + 2][LB + 3];
-          s[0][0] = sqrt(kPi * ip);
+      for (int d = 0; d < 3; ++d) {
+        const double xpa = P[d] - A[d], xpb = P[d] - B[d];
+        double s[LA + 2][LB + 3];
+        s[0][0] = sqrt(kPi * ip);
 #pragma unroll
-          for (int i = 0; i < LA + 1; ++i)
-            s[i + 1][0] = xpa * s[i][0] + (i > 0 ? i * 0.5 * ip * s[i > 0 ? i - 1 : 0][0] : 0.0);
+        for (int i = 0; i < LA + 1; ++i)
+          s[i + 1][0] = xpa * s[i][0] + (i > 0 ? i * 0.5 * ip * s[i > 0 ? i - 1 : 0][0] : 0.0);
 #pragma unroll
-          for (int j = 0; j < LB + 2; ++j)
-#pragma unroll
-            for (int i = 0; i <= LA + 1; ++i) {
-              double v = xpb * s[i][j];
-              if (i > 0) v += i * 0.5 * ip * s[i > 0 ? i - 1 : 0][j];
-              if (j > 0) v += j * 0.5 * ip * s[i][j > 0 ? j - 1 : 0];
-              s[i][j + 1] = v;
-            }
+        for (int j = 0; j < LB + 2; ++j)
 #pragma unroll
           for (int i = 0; i <= LA + 1; ++i) {
+            double v = xpb * s[i][j];
+            if (i > 0) v += i * 0.5 * ip * s[i > 0 ? i - 1 : 0][j];
+            if (j > 0) v += j * 0.5 * ip * s[i][j > 0 ? j - 1 : 0];
+            s[i][j + 1] = v;
+          }
 #pragma unroll
-            for (int j = 0; j < LB + 3; ++j) s1[d][i][j] = s[i][j];
+        for (int i = 0; i <= LA + 1; ++i) {
 #pragma unroll
-            for (int j = 0; j <= LB; ++j) {
-              double v = -2.0 * b * (2 * j + 1) * s[i][j] + 4.0 * b * b * s[i][j + 2];
-              if (j >= 2) v += j * (j - 1) * s[i][j >= 2 ? j - 2 : 0];
-              t1[d][i][j] = -0.5 * v;
-            }
+          for (int j = 0; j < LB + 3; ++j) s1[d][i][j] = s[i][j];
+#pragma unroll
+          for (int j = 0; j <= LB; ++j) {
+            double v = -2.0 * b * (2 * j + 1) * s[i][j] + 4.0 * b * b * s[i][j + 2];
+            if (j >= 2) v += j * (j - 1) * s[i][j >= 2 ? j - 2 : 0];
+            t1[d][i][j] = -0.5 * v;
           }
         }
+      }
+#pragma unroll
+      for (int i = 0; i < NCA; ++i)
+#pragma unroll
+        for (int j = 0; j < NCB; ++j) {
+          const int ax = ca.x[i], ay = ca.y[i], az = ca.z[i];
+          const int bx = cb.x[j], by = cb.y[j], bz = cb.z[j];
+          const double sx = s1[0][ax][bx], sy = s1[1][ay][by], sz = s1[2][az][bz];
+          const double tx = t1[0][ax][bx], ty = t1[1][ay][by], tz = t1[2][az][bz];
+          // derivative tables along each direction
+          const double dsx = 2.0 * a * s1[0][ax + 1][bx] - (ax ? ax * s1[0][ax ? ax - 1 : 0][bx] : 0.0);
+          const double dsy = 2.0 * a * s1[1][ay + 1][by] - (ay ? ay * s1[1][ay ? ay - 1 : 0][by] : 0.0);
+          const double dsz = 2.0 * a * s1[2][az + 1][bz] - (az ? az * s1[2][az ? az - 1 : 0][bz] : 0.0);
+          const double dtx = 2.0 * a * t1[0][ax + 1][bx] - (ax ? ax * t1[0][ax ? ax - 1 : 0][bx] : 0.0);
+          const double dty = 2.0 * a * t1[1][ay + 1][by] - (ay ? ay * t1[1][ay ? ay - 1 : 0][by] : 0.0);
+          const double dtz = 2.0 * a * t1[2][az + 1][bz] - (az ? az * t1[2][az ? az - 1 : 0][bz] : 0.0);
+          const double wd = kab * dc[i][j], wo = kab * wc[i][j];
+          // dS/dA_x = dsx sy sz ; dT/dA_x = dtx sy sz + dsx (ty sz + sy tz)
+          gst[0] += wd * (dtx * sy * sz + dsx * (ty * sz + sy * tz)) - wo * dsx * sy * sz;
+          gst[1] += wd * (dty * sx * sz + dsy * (tx * sz + sx * tz)) - wo * sx * dsy * sz;
+          gst[2] += wd * (dtz * sx * sy + dsz * (tx * sy + sx * ty)) - wo * sx * sy * dsz;
+        }
+    }
+  // nuclear attraction: basis-centre derivatives; the nucleus gets -(A+B)
+  for (int c = ln.c0; c < mol.natom; c += ln.dc) {
+    const int atomC = mol.atom_off + c;
+    const double* Cn = xyz + 3 * atomC;
+    const double zc = charge[atomC];
+    double cA[3] = {0.0, 0.0, 0.0}, cB[3] = {0.0, 0.0, 0.0};
+    for (int k = ln.k0; k < nab; k += ln.dk) {
+      const int ia = pa0 + k / nb, ib = pb0 + k % nb;
+      const double a = orb.exps[ia], b = orb.exps[ib];
+      const double p = a + b, ip = 1.0 / p;
+      const double kab = exp(-a * b * ip * rab2) * orb.coefs[ia] * orb.coefs[ib];
+      const double P[3] = {(a * A[0] + b * B[0]) * ip, (a * A[1] + b * B[1]) * ip,
+                           (a * A[2] + b * B[2]) * ip};
+      const double vpref = 2.0 * kPi * ip * kab;
+      const double PC[3] = {P[0] - Cn[0], P[1] - Cn[1], P[2] - Cn[2]};
+      const double tt = p * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]);
+      double u[NR], w[NR];
+      rys_roots<NR>(tt, u, w);
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        const double ur = u[r];
+        const double b10 = 0.5 * ip * (1.0 - ur);
+        double ix[LA + 2][LB + 2], iy[LA + 2][LB + 2], iz[LA + 2][LB + 2];
+        rys_2d<LA + 1, LB + 1, 0>(P[0] - A[0] - ur * PC[0], 0.0, b10, 0.0, 0.0, ab[0], 0, ix);
+        rys_2d<LA + 1, LB + 1, 0>(P[1] - A[1] - ur * PC[1], 0.0, b10, 0.0, 0.0, ab[1], 0, iy);
+        rys_2d<LA + 1, LB + 1, 0>(P[2] - A[2] - ur * PC[2], 0.0, b10, 0.0, 0.0, ab[2], 0, iz);
+        const double wr = -zc * vpref * w[r];
 #pragma unroll
         for (int i = 0; i < NCA; ++i)
 #pragma unroll
           for (int j = 0; j < NCB; ++j) {
             const int ax = ca.x[i], ay = ca.y[i], az = ca.z[i];
             const int bx = cb.x[j], by = cb.y[j], bz = cb.z[j];
-            const double sx = s1[0][ax][bx], sy = s1[1][ay][by], sz = s1[2][az][bz];
-            const double tx = t1[0][ax][bx], ty = t1[1][ay][by], tz = t1[2][az][bz];
-            // derivative tables along each direction
-            const double dsx = 2.0 * a * s1[0][ax + 1][bx] - (ax ? ax * s1[0][ax ? ax - 1 : 0][bx] : 0.0);
-            const double dsy = 2.0 * a * s1[1][ay + 1][by] - (ay ? ay * s1[1][ay ? ay - 1 : 0][by] : 0.0);
-            const double dsz = 2.0 * a * s1[2][az + 1][bz] - (az ? az * s1[2][az ? az - 1 : 0][bz] : 0.0);
-            const double dtx = 2.0 * a * t1[0][ax + 1][bx] - (ax ? ax * t1[0][ax ? ax - 1 : 0][bx] : 0.0);
-            const double dty = 2.0 * a * t1[1][ay + 1][by] - (ay ? ay * t1[1][ay ? ay - 1 : 0][by] : 0.0);
-            const double dtz = 2.0 * a * t1[2][az + 1][bz] - (az ? az * t1[2][az ? az - 1 : 0][bz] : 0.0);
-            const double wd = kab * dc[i][j], wo = kab * wc[i][j];
-            // dS/dA_x = dsx sy sz ; dT/dA_x = dtx sy sz + dsx (ty sz + sy tz)
-            gst[0] += wd * (dtx * sy * sz + dsx * (ty * sz + sy * tz)) - wo * dsx * sy * sz;
-            gst[1] += wd * (dty * sx * sz + dsy * (tx * sz + sx * tz)) - wo * sx * dsy * sz;
-            gst[2] += wd * (dtz * sx * sy + dsz * (tx * sy + sx * ty)) - wo * sx * sy * dsz;
+            const double x0 = ix[ax][bx], y0 = iy[ay][by], z0 = iz[az][bz];
+            const double dax = 2.0 * a * ix[ax + 1][bx] - (ax ? ax * ix[ax ? ax - 1 : 0][bx] : 0.0);
+            const double day = 2.0 * a * iy[ay + 1][by] - (ay ? ay * iy[ay ? ay - 1 : 0][by] : 0.0);
+            const double daz = 2.0 * a * iz[az + 1][bz] - (az ? az * iz[az ? az - 1 : 0][bz] : 0.0);
+            const double dbx = 2.0 * b * ix[ax][bx + 1] - (bx ? bx * ix[ax][bx ? bx - 1 : 0] : 0.0);
+            const double dby = 2.0 * b * iy[ay][by + 1] - (by ? by * iy[ay][by ? by - 1 : 0] : 0.0);
+            const double dbz = 2.0 * b * iz[az][bz + 1] - (bz ? bz * iz[az][bz ? bz - 1 : 0] : 0.0);
+            const double wd = wr * dc[i][j];
+            cA[0] = fma(wd, dax * y0 * z0, cA[0]);
+            cA[1] = fma(wd, x0 * day * z0, cA[1]);
+            cA[2] = fma(wd, x0 * y0 * daz, cA[2]);
+            cB[0] = fma(wd, dbx * y0 * z0, cB[0]);
+            cB[1] = fma(wd, x0 * dby * z0, cB[1]);
+            cB[2] = fma(wd, x0 * y0 * dbz, cB[2]);
           }
       }
-      // nuclear attraction: basis-centre derivatives; the nucleus gets -(A+B)
-      const double vpref = 2.0 * kPi * ip * kab;
-      for (int c = 0; c < mol.natom; ++c) {
-        const int atomC = mol.atom_off + c;
-        const double* Cn = xyz + 3 * atomC;
-        const double zc = charge[atomC];
-        const double PC[3] = {P[0] - Cn[0], P[1] - Cn[1], P[2] - Cn[2]};
-        const double tt = p * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]);
-        double u[NR], w[NR];
-        rys_roots<NR>(tt, u, w);
-        double cA[3] = {0.0, 0.0, 0.0}, cB[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int r = 0; r < NR; ++r) {
-          const double ur = u[r];
-          const double b10 = 0.5 * ip * (1.0 - ur);
-          double ix[LA + 2][LB + 2], iy[LA + 2][LB + 2], iz[LA + 2][LB + 2];
-          rys_2d<LA + 1, LB + 1, 0>(P[0] - A[0] - ur * PC[0], 0.0, b10, 0.0, 0.0, ab[0], 0, ix);
-          rys_2d<LA + 1, LB + 1, 0>(P[1] - A[1] - ur * PC[1], 0.0, b10, 0.0, 0.0, ab[1], 0, iy);
-          rys_2d<LA + 1, LB + 1, 0>(P[2] - A[2] - ur * PC[2], 0.0, b10, 0.0, 0.0, ab[2], 0, iz);
-          const double wr = -zc * vpref * w[r];
-#pragma unroll
-          for (int i = 0; i < NCA; ++i)
-#pragma unroll
-            for (int j = 0; j < NCB; ++j) {
-              const int ax = ca.x[i], ay = ca.y[i], az = ca.z[i];
-              const int bx = cb.x[j], by = cb.y[j], bz = cb.z[j];
-              const double x0 = ix[ax][bx], y0 = iy[ay][by], z0 = iz[az][bz];
-              const double dax = 2.0 * a * ix[ax + 1][bx] - (ax ? ax * ix[ax ? ax - 1 : 0][bx] : 0.0);
-              const double day = 2.0 * a * iy[ay + 1][by] - (ay ? ay * iy[ay ? ay - 1 : 0][by] : 0.0);
-              const double daz = 2.0 * a * iz[az + 1][bz] - (az ? az * iz[az ? az - 1 : 0][bz] : 0.0);
-              const double dbx = 2.0 * b * ix[ax][bx + 1] - (bx ? bx * ix[ax][bx ? bx - 1 : 0] : 0.0);
-              const double dby = 2.0 * b * iy[ay][by + 1] - (by ? by * iy[ay][by ? by - 1 : 0] : 0.0);
-              const double dbz = 2.0 * b * iz[az][bz + 1] - (bz ? bz * iz[az][bz ? bz - 1 : 0] : 0.0);
-              const double wd = wr * dc[i][j];
-              cA[0] = fma(wd, dax * y0 * z0, cA[0]);
-              cA[1] = fma(wd, x0 * day * z0, cA[1]);
-              cA[2] = fma(wd, x0 * y0 * daz, cA[2]);
-              cB[0] = fma(wd, dbx * y0 * z0, cB[0]);
-              cB[1] = fma(wd, x0 * dby * z0, cB[1]);
-              cB[2] = fma(wd, x0 * y0 * dbz, cB[2]);
-            }
-        }
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          gvA[d] += cA[d];
-          gvB[d] += cB[d];
-          atomicAdd(grad + 3 * atomC + d, -(cA[d] + cB[d]));
-        }
-      }
     }
+    if (nab)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        gvA[d] += cA[d];
+        gvB[d] += cB[d];
+        add(3 * atomC + d, -(cA[d] + cB[d]));
+      }
   }
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    atomicAdd(grad + 3 * atomA + d, gst[d] + gvA[d]);
-    atomicAdd(grad + 3 * atomB + d, -gst[d] + gvB[d]);
+    double ga = gst[d] + gvA[d], gb = gvB[d] - gst[d];
+#pragma unroll
+    for (int off = 1; off < k1eLanes; off <<= 1) {
+      ga += __shfl_xor_sync(0xffffffffu, ga, off);
+      gb += __shfl_xor_sync(0xffffffffu, gb, off);
+    }
+    if (valid && ln.lane == 0) {
+      add(3 * atomA + d, ga);
+      add(3 * atomB + d, gb);
+    }
   }
+  if (local) flush_sums(sums, mol, grad);
 }
 
 // ---------------------------------------------------------------------------
@@ -706,7 +735,7 @@ static void glaunch2(const ClassLaunch& cl, const KernelArgs& k, cudaStream_t st
 
 template <int LA, int LB, bool SPH>
 static void glaunch1(const ClassLaunch& cl, const KernelArgs& k, cudaStream_t st) {
-  grad1e_kernel<LA, LB, SPH><<<cl.nblocks, 128, 0, st>>>(k.orb, k.xyz, k.charge, k.mols, cl.pairs,
+  grad1e_kernel<LA, LB, SPH><<<cl.nblocks * k1eLanes, 128, 0, st>>>(k.orb, k.xyz, k.charge, k.mols, cl.pairs,
                                                           cl.cms, cl.ncm, k.w1, k.w2, k.grad);
 }
 

@@ -421,6 +421,19 @@ __device__ __forceinline__ void store_1e(int mode, const double (&acc)[ncart(LA)
     }
 }
 
+// sum over the lanes of a pair (k1eLanes consecutive lanes), in every lane
+template <int NCA, int NCB>
+__device__ __forceinline__ void lanes_sum(double (&acc)[NCA][NCB]) {
+#pragma unroll
+  for (int i = 0; i < NCA; ++i)
+#pragma unroll
+    for (int j = 0; j < NCB; ++j)
+#pragma unroll
+      for (int off = 1; off < k1eLanes; off <<= 1) acc[i][j] += __shfl_xor_sync(0xffffffffu, acc[i][j], off);
+}
+
+// k1eLanes lanes per shell pair: they share its primitive pairs for S and T,
+// and its (primitive pair, nucleus) products for V (Lanes1e)
 template <int LA, int LB, bool SPH>
 __global__ void __launch_bounds__(128)
     int1e_kernel(DevBasis orb, const double* __restrict__ xyz, const double* __restrict__ charge,
@@ -433,104 +446,122 @@ __global__ void __launch_bounds__(128)
   constexpr int MODE = SPH ? 0 : 1;
   constexpr Cart<LA> ca{};
   constexpr Cart<LB> cb{};
-  const ClassMol cm = cms[find_cm(cms, ncm, blockIdx.x)];
-  const int t = (blockIdx.x - cm.chunk_begin) * 128 + threadIdx.x;
-  if (t >= cm.ntriples) return;
+  const int chunk = blockIdx.x / k1eLanes;
+  const ClassMol cm = cms[find_cm(cms, ncm, chunk)];
+  const int t = (chunk - cm.chunk_begin) * 128 +
+                ((blockIdx.x % k1eLanes) * 128 + threadIdx.x) / k1eLanes;
+  const bool valid = t < cm.ntriples;
   const DevMol mol = mols[cm.mol];
-  const int2 pr = pairs[cm.pair_begin + t];
+  const Lanes1e ln(mol.natom);
+  const int2 pr = pairs[cm.pair_begin + (valid ? t : 0)];
   const double* A = xyz + 3 * orb.atom[pr.x];
   const double* B = xyz + 3 * orb.atom[pr.y];
   const double ab[3] = {A[0] - B[0], A[1] - B[1], A[2] - B[2]};
   const double rab2 = ab[0] * ab[0] + ab[1] * ab[1] + ab[2] * ab[2];
-  const int pa0 = orb.prim_off[pr.x], na = orb.nprim[pr.x];
+  const int pa0 = orb.prim_off[pr.x];
   const int pb0 = orb.prim_off[pr.y], nb = orb.nprim[pr.y];
-  double accs[NCA][NCB], acct[NCA][NCB], accv[NCA][NCB];
+  const int nab = valid ? orb.nprim[pr.x] * nb : 0;
+  double accs[NCA][NCB], acct[NCA][NCB];
 #pragma unroll
   for (int i = 0; i < NCA; ++i)
 #pragma unroll
-    for (int j = 0; j < NCB; ++j) accs[i][j] = acct[i][j] = accv[i][j] = 0.0;
-  for (int ia = 0; ia < na; ++ia) {
-    const double a = orb.exps[pa0 + ia], ca_ = orb.coefs[pa0 + ia];
-    for (int ib = 0; ib < nb; ++ib) {
-      const double b = orb.exps[pb0 + ib], cb_ = orb.coefs[pb0 + ib];
-      const double p = a + b, ip = 1.0 / p;
-      const double kab = exp(-a * b * ip * rab2) * ca_ * cb_;
-      const double P[3] = {(a * A[0] + b * B[0]) * ip, (a * A[1] + b * B[1]) * ip,
-                           (a * A[2] + b * B[2]) * ip};
-      // overlap/kinetic 1-D tables
-      double s1[3][LA + 1][LB + 3], t1[3][LA + 1][LB + 1];
+    for (int j = 0; j < NCB; ++j) accs[i][j] = acct[i][j] = 0.0;
+  for (int k = ln.lane; k < nab; k += k1eLanes) {
+    const int ia = pa0 + k / nb, ib = pb0 + k % nb;
+    const double a = orb.exps[ia], b = orb.exps[ib];
+    const double p = a + b, ip = 1.0 / p;
+    const double kab = exp(-a * b * ip * rab2) * orb.coefs[ia] * orb.coefs[ib];
+    // overlap/kinetic 1-D tables
+    double s1[3][LA + 1][LB + 3], t1[3][LA + 1][LB + 1];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const double xpa = P[d] - A[d], xpb = P[d] - B[d];
-        double s[LA + 1][LB + 3];
-        s[0][0] = sqrt(kPi * ip);
+    for (int d = 0; d < 3; ++d) {
+      const double P = (a * A[d] + b * B[d]) * ip;
+      const double xpa = P - A[d], xpb = P - B[d];
+      double s[LA + 1][LB + 3];
+      s[0][0] = sqrt(kPi * ip);
 #pragma unroll
-        for (int i = 0; i < LA; ++i)
-          s[i + 1][0] = xpa * s[i][0] + (i > 0 ? i * 0.5 * ip * s[i > 0 ? i - 1 : 0][0] : 0.0);
+      for (int i = 0; i < LA; ++i)
+        s[i + 1][0] = xpa * s[i][0] + (i > 0 ? i * 0.5 * ip * s[i > 0 ? i - 1 : 0][0] : 0.0);
 #pragma unroll
-        for (int j = 0; j < LB + 2; ++j)
-#pragma unroll
-          for (int i = 0; i <= LA; ++i) {
-            double v = xpb * s[i][j];
-            if (i > 0) v += i * 0.5 * ip * s[i > 0 ? i - 1 : 0][j];
-            if (j > 0) v += j * 0.5 * ip * s[i][j > 0 ? j - 1 : 0];
-            s[i][j + 1] = v;
-          }
+      for (int j = 0; j < LB + 2; ++j)
 #pragma unroll
         for (int i = 0; i <= LA; ++i) {
-#pragma unroll
-          for (int j = 0; j < LB + 3; ++j) s1[d][i][j] = s[i][j];
-#pragma unroll
-          for (int j = 0; j <= LB; ++j) {
-            double v = -2.0 * b * (2 * j + 1) * s[i][j] + 4.0 * b * b * s[i][j + 2];
-            if (j >= 2) v += j * (j - 1) * s[i][j >= 2 ? j - 2 : 0];
-            t1[d][i][j] = -0.5 * v;
-          }
+          double v = xpb * s[i][j];
+          if (i > 0) v += i * 0.5 * ip * s[i > 0 ? i - 1 : 0][j];
+          if (j > 0) v += j * 0.5 * ip * s[i][j > 0 ? j - 1 : 0];
+          s[i][j + 1] = v;
         }
-      }
 #pragma unroll
-      for (int i = 0; i < NCA; ++i)
+      for (int i = 0; i <= LA; ++i) {
 #pragma unroll
-        for (int j = 0; j < NCB; ++j) {
-          const double sx = s1[0][ca.x[i]][cb.x[j]], sy = s1[1][ca.y[i]][cb.y[j]],
-                       sz = s1[2][ca.z[i]][cb.z[j]];
-          accs[i][j] = fma(kab, sx * sy * sz, accs[i][j]);
-          acct[i][j] = fma(kab,
-                           t1[0][ca.x[i]][cb.x[j]] * sy * sz + sx * t1[1][ca.y[i]][cb.y[j]] * sz +
-                               sx * sy * t1[2][ca.z[i]][cb.z[j]],
-                           acct[i][j]);
-        }
-      // nuclear attraction, every nucleus of the molecule
-      const double vpref = 2.0 * kPi * ip * kab;
-      for (int c = 0; c < mol.natom; ++c) {
-        const double* Cn = xyz + 3 * (mol.atom_off + c);
-        const double zc = charge[mol.atom_off + c];
-        const double PC[3] = {P[0] - Cn[0], P[1] - Cn[1], P[2] - Cn[2]};
-        const double tt = p * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]);
-        double u[NR], w[NR];
-        rys_roots<NR>(tt, u, w);
+        for (int j = 0; j < LB + 3; ++j) s1[d][i][j] = s[i][j];
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-          const double ur = u[r];
-          const double b10 = 0.5 * ip * (1.0 - ur);
-          double ix[LA + 1][LB + 1], iy[LA + 1][LB + 1], iz[LA + 1][LB + 1];
-          rys_2d<LA, LB, 0>(P[0] - A[0] - ur * PC[0], 0.0, b10, 0.0, 0.0, ab[0], 0, ix);
-          rys_2d<LA, LB, 0>(P[1] - A[1] - ur * PC[1], 0.0, b10, 0.0, 0.0, ab[1], 0, iy);
-          rys_2d<LA, LB, 0>(P[2] - A[2] - ur * PC[2], 0.0, b10, 0.0, 0.0, ab[2], 0, iz);
-          const double wr = -zc * vpref * w[r];
-#pragma unroll
-          for (int i = 0; i < NCA; ++i)
-#pragma unroll
-            for (int j = 0; j < NCB; ++j)
-              accv[i][j] = fma(wr * ix[ca.x[i]][cb.x[j]],
-                               iy[ca.y[i]][cb.y[j]] * iz[ca.z[i]][cb.z[j]], accv[i][j]);
+        for (int j = 0; j <= LB; ++j) {
+          double v = -2.0 * b * (2 * j + 1) * s[i][j] + 4.0 * b * b * s[i][j + 2];
+          if (j >= 2) v += j * (j - 1) * s[i][j >= 2 ? j - 2 : 0];
+          t1[d][i][j] = -0.5 * v;
         }
       }
     }
+#pragma unroll
+    for (int i = 0; i < NCA; ++i)
+#pragma unroll
+      for (int j = 0; j < NCB; ++j) {
+        const double sx = s1[0][ca.x[i]][cb.x[j]], sy = s1[1][ca.y[i]][cb.y[j]],
+                     sz = s1[2][ca.z[i]][cb.z[j]];
+        accs[i][j] = fma(kab, sx * sy * sz, accs[i][j]);
+        acct[i][j] = fma(kab,
+                         t1[0][ca.x[i]][cb.x[j]] * sy * sz + sx * t1[1][ca.y[i]][cb.y[j]] * sz +
+                             sx * sy * t1[2][ca.z[i]][cb.z[j]],
+                         acct[i][j]);
+      }
   }
-  store_1e<LA, LB, NOA, NOB>(MODE, accs, orb, pr, mol, S);
-  store_1e<LA, LB, NOA, NOB>(MODE, acct, orb, pr, mol, T);
-  store_1e<LA, LB, NOA, NOB>(MODE, accv, orb, pr, mol, V);
+  lanes_sum(accs);
+  lanes_sum(acct);
+  if (valid && ln.lane == 0) store_1e<LA, LB, NOA, NOB>(MODE, accs, orb, pr, mol, S);
+  if (valid && ln.lane == 1) store_1e<LA, LB, NOA, NOB>(MODE, acct, orb, pr, mol, T);
+
+  // nuclear attraction, every nucleus of the molecule
+  double accv[NCA][NCB];
+#pragma unroll
+  for (int i = 0; i < NCA; ++i)
+#pragma unroll
+    for (int j = 0; j < NCB; ++j) accv[i][j] = 0.0;
+  for (int k = ln.k0; k < nab; k += ln.dk) {
+    const int ia = pa0 + k / nb, ib = pb0 + k % nb;
+    const double a = orb.exps[ia], b = orb.exps[ib];
+    const double p = a + b, ip = 1.0 / p;
+    const double kab = exp(-a * b * ip * rab2) * orb.coefs[ia] * orb.coefs[ib];
+    const double P[3] = {(a * A[0] + b * B[0]) * ip, (a * A[1] + b * B[1]) * ip,
+                         (a * A[2] + b * B[2]) * ip};
+    const double vpref = 2.0 * kPi * ip * kab;
+    for (int c = ln.c0; c < mol.natom; c += ln.dc) {
+      const double* Cn = xyz + 3 * (mol.atom_off + c);
+      const double zc = charge[mol.atom_off + c];
+      const double PC[3] = {P[0] - Cn[0], P[1] - Cn[1], P[2] - Cn[2]};
+      const double tt = p * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]);
+      double u[NR], w[NR];
+      rys_roots<NR>(tt, u, w);
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        const double ur = u[r];
+        const double b10 = 0.5 * ip * (1.0 - ur);
+        double ix[LA + 1][LB + 1], iy[LA + 1][LB + 1], iz[LA + 1][LB + 1];
+        rys_2d<LA, LB, 0>(P[0] - A[0] - ur * PC[0], 0.0, b10, 0.0, 0.0, ab[0], 0, ix);
+        rys_2d<LA, LB, 0>(P[1] - A[1] - ur * PC[1], 0.0, b10, 0.0, 0.0, ab[1], 0, iy);
+        rys_2d<LA, LB, 0>(P[2] - A[2] - ur * PC[2], 0.0, b10, 0.0, 0.0, ab[2], 0, iz);
+        const double wr = -zc * vpref * w[r];
+#pragma unroll
+        for (int i = 0; i < NCA; ++i)
+#pragma unroll
+          for (int j = 0; j < NCB; ++j)
+            accv[i][j] = fma(wr * ix[ca.x[i]][cb.x[j]],
+                             iy[ca.y[i]][cb.y[j]] * iz[ca.z[i]][cb.z[j]], accv[i][j]);
+      }
+    }
+  }
+  lanes_sum(accv);
+  if (valid && ln.lane == 0) store_1e<LA, LB, NOA, NOB>(MODE, accv, orb, pr, mol, V);
 }
 
 // ---------------------------------------------------------------------------
@@ -556,7 +587,7 @@ static void launch2(const ClassLaunch& cl, const KernelArgs& k, cudaStream_t st)
 
 template <int LA, int LB, bool SPH>
 static void launch1(const ClassLaunch& cl, const KernelArgs& k, cudaStream_t st) {
-  int1e_kernel<LA, LB, SPH><<<cl.nblocks, 128, 0, st>>>(k.orb, k.xyz, k.charge, k.mols, cl.pairs,
+  int1e_kernel<LA, LB, SPH><<<cl.nblocks * k1eLanes, 128, 0, st>>>(k.orb, k.xyz, k.charge, k.mols, cl.pairs,
                                                         cl.cms, cl.ncm, k.out, k.out2, k.out3);
 }
 

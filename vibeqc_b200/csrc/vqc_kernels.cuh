@@ -197,6 +197,24 @@ __device__ __forceinline__ int find_cm(const ClassMol* __restrict__ cms, int ncm
   return n - 1;
 }
 
+// One-electron kernels: k1eLanes lanes per shell pair.  With one thread per
+// pair a class of contracted pairs was a few hundred warps, each a serial
+// chain over primitive pairs times nuclei (5 % of the resident-warp limit,
+// FP64 pipe 4 % active).  The lanes split the nuclei; with fewer nuclei than
+// lanes, the primitive pairs as well.  (ss) derivatives of 12 x (H2O)6 0.290 ->
+// 0.068 ms, (ps) 0.245 -> 0.082; (ss) values of 8 x (H2O)9 0.151 -> 0.056.
+constexpr int k1eLanes = 8;
+struct Lanes1e {
+  int lane, c0, dc, k0, dk;
+  __device__ __forceinline__ explicit Lanes1e(int natom) {
+    lane = threadIdx.x % k1eLanes;
+    dc = natom <= 1 ? 1 : (natom <= 2 ? 2 : (natom <= 4 ? 4 : 8));
+    dk = k1eLanes / dc;
+    c0 = lane % dc;
+    k0 = lane / dc;
+  }
+};
+
 bool dispatch_int3c(const ClassLaunch& cl, const KernelArgs& k, bool sph, cudaStream_t st);
 bool dispatch_int2c(const ClassLaunch& cl, const KernelArgs& k, bool sph, cudaStream_t st);
 bool dispatch_int1e(const ClassLaunch& cl, const KernelArgs& k, bool sph, cudaStream_t st);
