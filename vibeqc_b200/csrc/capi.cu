@@ -61,6 +61,24 @@ static int upload(DeviceBuffers& owned, const std::vector<T>& h, T** d) {
   return VQC_STATUS_SUCCESS;
 }
 
+bool SideStreams::ensure() {
+  if (ready) return true;
+  bool ok = fork || cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) == cudaSuccess;
+  for (int i = 0; ok && i < kStreams; ++i)
+    ok = (stream[i] || cudaStreamCreateWithFlags(&stream[i], cudaStreamNonBlocking) == cudaSuccess) &&
+         (join[i] || cudaEventCreateWithFlags(&join[i], cudaEventDisableTiming) == cudaSuccess);
+  if (!ok) cudaGetLastError();
+  return ready = ok;
+}
+
+SideStreams::~SideStreams() {
+  if (fork) cudaEventDestroy(fork);
+  for (int i = 0; i < kStreams; ++i) {
+    if (join[i]) cudaEventDestroy(join[i]);
+    if (stream[i]) cudaStreamDestroy(stream[i]);
+  }
+}
+
 Plan::~Plan() {
   for (void* p : owned) cudaFree(p);
 }
@@ -326,17 +344,49 @@ int vqc_plan_molecule(const vqc_plan* plan, int32_t index, vqc_molecule_info* in
   return VQC_STATUS_SUCCESS;
 }
 
+// The class kernels of a list are independent of each other (distinct outputs,
+// or atomic sums), and one class alone fills the GPU only for large batches:
+// those of one small molecule are a few CTAs that wait on latency, and every
+// class has a tail.  They run round robin over the caller's stream and the
+// plan's side streams, which start after the caller's earlier work and are
+// joined before the call returns to it.  Under stream capture (the side
+// streams would stay in the capture) and while another thread uses the plan's
+// streams, they run in order on the caller's stream.
+// In order -> side by side: 8 x (H2O)9 integrals 4.39 -> 4.10 ms, 12 x (H2O)6
+// derivatives 4.37 -> 3.71, J, K and gradient of one (H2O)7 6.21 -> 5.73.
 static int run_classes(Plan* p, const std::vector<ClassLaunch>& list,
                        bool (*dispatch)(const ClassLaunch&, const KernelArgs&, bool, cudaStream_t),
                        const KernelArgs& k, cudaStream_t st, const char* what) {
+  SideStreams& side = p->side;
+  std::unique_lock<std::mutex> lock(side.busy, std::try_to_lock);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+  bool fan = list.size() > 2 && lock.owns_lock() &&
+             cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
+             capture == cudaStreamCaptureStatusNone && side.ensure();
+  const int used = fan ? (int)std::min<size_t>(SideStreams::kStreams, list.size() - 1) : 0;
+  cudaError_t e = cudaSuccess;
+  if (used && !(e = cudaEventRecord(side.fork, st)))
+    for (int i = 0; i < used && !e; ++i) e = cudaStreamWaitEvent(side.stream[i], side.fork, 0);
+  if (e) return cuda_status(e, what);
+  int status = VQC_STATUS_SUCCESS;
+  int next = 0;
   for (const ClassLaunch& cl : list) {
-    if (!dispatch(cl, k, p->sph, st))
-      return fail(VQC_STATUS_INVALID_ARGUMENT, std::string(what) + ": unsupported class");
+    if (!dispatch(cl, k, p->sph, next ? side.stream[next - 1] : st)) {
+      status = fail(VQC_STATUS_INVALID_ARGUMENT, std::string(what) + ": unsupported class");
+      break;
+    }
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_status(e, what);
+    if ((e = cudaGetLastError())) {
+      status = cuda_status(e, what);
+      break;
+    }
+    next = next == used ? 0 : next + 1;
   }
-  return VQC_STATUS_SUCCESS;
+  for (int i = 0; i < used; ++i) {  // on errors too: what was launched stays ordered
+    if (!(e = cudaEventRecord(side.join[i], side.stream[i]))) e = cudaStreamWaitEvent(st, side.join[i], 0);
+    if (e && status == VQC_STATUS_SUCCESS) status = cuda_status(e, what);
+  }
+  return status;
 }
 
 int vqc_int1e(vqc_plan* plan, const double* xyz, double* s, double* t, double* v, void* stream) {

@@ -1,6 +1,7 @@
 // Host-side plan object behind the opaque vqc_plan handle.
 #pragma once
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -15,6 +16,20 @@ using DeviceBuffers = std::vector<void*>;
 
 struct HostShells {
   std::vector<int> l, atom, nprim, prim_off, func_off;
+};
+
+// Streams and events over which a plan's class kernels run side by side.  They
+// belong to the plan and are used by one call at a time (the mutex is held
+// while a call enqueues); a call that finds them taken runs on its own stream.
+struct SideStreams {
+  static constexpr int kStreams = 3;  // beside the caller's
+  std::mutex busy;
+  cudaStream_t stream[kStreams] = {};
+  cudaEvent_t fork = nullptr, join[kStreams] = {};
+  bool ready = false;
+
+  bool ensure();
+  ~SideStreams();
 };
 
 struct Plan {
@@ -47,6 +62,7 @@ struct Plan {
   std::vector<int> mol_shell_off;
   DevMol* dtile_mol = nullptr;
   ClassMol* dtile_cms = nullptr;
+  SideStreams side;
 
   int build(const vqc_batch_desc& d);
   ~Plan();
