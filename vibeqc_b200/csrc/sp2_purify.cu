@@ -51,6 +51,13 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
+// Once |tr X - tr X^2| < tol, kPolish more steps, X^2 and then 2X - X^2: they
+// square the distance of every eigenvalue from 0 and from 1, so the projector
+// is idempotent to rounding instead of to whatever below tol the last step
+// happened to reach (the distance from eigenvectors scattered over 1e-14 to
+// 5e-13 with it), for 4 % of the steps.
+constexpr int kPolish = 2;
+
 // the smaller of |tr X^2 - n_occ| and |tr(2X - X^2) - n_occ| picks the step
 __device__ __forceinline__ bool take_square(double tr, double tr2, double nocc) {
   return fabs(tr2 - nocc) < fabs(2.0 * tr - tr2 - nocc);
@@ -130,7 +137,7 @@ __global__ void __launch_bounds__(kSmallThreads)
     }
   const int nt = (np + 15) / 16, ntiles = nt * (nt + 1) / 2;
   const int fr = lane >> 2, fc = lane & 3;
-  int cur = 0;
+  int cur = 0, polish = 0;
   for (int step = 0;; ++step) {
     tr = warp_sum(tr);
     fro = warp_sum(fro);
@@ -145,8 +152,9 @@ __global__ void __launch_bounds__(kSmallThreads)
       tr += rp[w];
       fro += rp[kSmallWarps + w];
     }
-    if (fabs(tr - fro) < tol || step >= max_steps) break;
-    const bool square = take_square(tr, fro, nocc);
+    if (polish || fabs(tr - fro) < tol) ++polish;
+    if (polish > kPolish || (!polish && step >= max_steps)) break;
+    const bool square = polish ? polish == 1 : take_square(tr, fro, nocc);
     const double* x = sm + cur * bufs;
     double* xn = sm + (cur ^ 1) * bufs;
     tr = fro = 0.0;
@@ -349,14 +357,15 @@ __global__ void __launch_bounds__(GroupCfg<BM>::THREADS, GroupCfg<BM>::CTAS)
         fro = fma(v, v, fro);
         if (i == j) tr += v;
       }
-    int cur = 0;
+    int cur = 0, polish = 0;
     for (int step = 0;; ++step) {
       publish(tr, fro);
       arrived += G;
       if (!group_barrier(count, arrived, p.error, &flag)) return;
       totals(tr, fro);
-      if (fabs(tr - fro) < p.tol || step >= p.max_steps) break;
-      const bool square = take_square(tr, fro, p.nocc);
+      if (polish || fabs(tr - fro) < p.tol) ++polish;
+      if (polish > kPolish || (!polish && step >= p.max_steps)) break;
+      const bool square = polish ? polish == 1 : take_square(tr, fro, p.nocc);
       const double* x = xbase + cur * xsize;
       double* xn = xbase + (cur ^ 1) * xsize;
       tr = fro = 0.0;
