@@ -1,0 +1,50 @@
+"""Layout kernels of the mixed J/K path at the edges of their tiles and vector forms."""
+
+import pytest
+import torch
+
+from vibeqc_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,x,ldq,shift", [
+    (1, 2, 4, 0), (9, 126, 128, 0), (64, 128, 128, 0), (5000, 116, 116, 0), (17, 130, 136, 0),
+    (33, 129, 132, 0), (12, 131, 131, 0), (7, 64, 64, 1)])  # odd x, unpadded rows, unaligned arrays
+def test_anchor_combine(rows, x, ldq, shift):
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    u0 = torch.randn(rows * x + shift, generator=g, device="cuda", dtype=torch.float64)[shift:]
+    dh, dl = (scale * torch.randn(rows * ldq + shift, generator=g, device="cuda")[shift:]
+              for scale in (1e-2, 1e-6))
+    vh, vl = (torch.full((rows * ldq + shift,), 7.0, device="cuda")[shift:] for _ in range(2))
+    before = u0.clone()
+    st = torch.cuda.current_stream().cuda_stream
+    args = (rows, x, ldq)
+    _lib.call("vqc_anchor_combine", u0.data_ptr(), dh.data_ptr(), dl.data_ptr(), vh.data_ptr(),
+              vl.data_ptr(), *args, 0.5, 0, st)
+    assert torch.equal(u0, before)
+    du = (dh.double() + dl.double()).view(rows, ldq)[:, :x]
+    want = before.view(rows, x) + 0.5 * du
+    v = (vh.double() + vl.double()).view(rows, ldq)
+    # V is rounded to FP32 (2^-24) and split into two TF32 parts (2^-22 of the value)
+    assert ((v[:, :x] - want).abs() <= 2.0**-21 * want.abs()).all()
+    assert (vh.view(rows, ldq)[:, x:] == 0).all() and (vl.view(rows, ldq)[:, x:] == 0).all()
+    _lib.call("vqc_anchor_combine", u0.data_ptr(), dh.data_ptr(), dl.data_ptr(), 0, 0, *args, 1.0, 1, st)
+    # one FP64 product and sum
+    bound = 4e-16 * (before.abs().view(rows, x) + du.abs())
+    assert ((u0.view(rows, x) - (before.view(rows, x) + du)).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("nb,n,x,ld", [(1, 1, 1, 4), (2, 24, 116, 24), (1, 31, 33, 32),
+                                       (3, 33, 31, 36), (1, 130, 257, 160)])
+def test_unpack_aux_major(nb, n, x, ld):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    bp = torch.randn(nb, n * (n + 1) // 2, x, generator=g, device="cuda", dtype=torch.float64)
+    b = torch.full((nb, n, x, ld), 7.0, device="cuda")
+    _lib.call("vqc_unpack_aux_major", bp.data_ptr(), nb, n, x, ld, b.data_ptr(),
+              torch.cuda.current_stream().cuda_stream)
+    i = torch.arange(n, device="cuda")
+    hi, lo = torch.maximum(i[:, None], i), torch.minimum(i[:, None], i)
+    full = bp[:, hi * (hi + 1) // 2 + lo]  # (nb, mu, nu, Q)
+    assert torch.equal(b[..., :n], full.transpose(2, 3).float())
+    assert (b[..., n:] == 0).all()
