@@ -244,6 +244,32 @@ int vqc_sp2_purify(const double* fo, int32_t nmol, int32_t n, double nocc, doubl
                    int32_t* error, void* stream);
 
 /*
+ * Convergence test and bookkeeping of one SCF iteration over nmol molecules of
+ * one size: rms density change over the nspin spins, the criteria of the
+ * reference (src/scf/cuda/scf_convergence_policy.cuh:18-37; applied when
+ * may_converge), d, c, f of the molecules active in active_in copied to
+ * *_final, and d_new, c_new taken over into d, c where a molecule stays active.
+ * n*n and n*ncol blocks are contiguous; partial holds 32 doubles per molecule;
+ * active and e_old are read from *_in and written to *_out (distinct arrays).
+ * flags[0]: a molecule stays active; flags[1]: the residual of a molecule that
+ * was active exceeds loose_tolerance.
+ */
+typedef struct vqc_scf_record_args {
+  uint32_t struct_size;
+  int32_t nmol, n, ncol, nspin, iteration, may_converge, reserved;
+  double energy_tolerance, density_tolerance, commutator_tolerance, loose_tolerance, energy_roundoff;
+  const double *energy, *cmax, *e_old_in;
+  const int32_t* active_in;
+  double *e_old_out, *final_e, *final_de, *final_drms, *partial;
+  int32_t* active_out;
+  int64_t* iters;
+  int32_t *converged, *flags;
+  const double *d_new[2], *c_new[2], *f[2];
+  double *d[2], *c[2], *d_final[2], *c_final[2], *f_final[2];
+} vqc_scf_record_args;
+int vqc_scf_record(const vqc_scf_record_args* args, void* stream);
+
+/*
  * Mixed-precision J/K over the FP32 whitened tensor stored aux-major per AO
  * row: b_aux_major[mol][mu][Q][nu], row length ld_ao >= nao (ld_ao % 4 == 0;
  * the Coulomb and fitted-density kernels take ld_ao <= 512,

@@ -89,6 +89,24 @@ class DfGradientResources(ctypes.Structure):
     ]
 
 
+class ScfRecordArgs(ctypes.Structure):
+    """``vqc_scf_record_args``."""
+
+    _fields_ = [
+        ("struct_size", ctypes.c_uint32),
+        *[(f, ctypes.c_int32) for f in ("nmol", "n", "ncol", "nspin", "iteration", "may_converge",
+                                        "reserved")],
+        *[(f, ctypes.c_double) for f in ("energy_tolerance", "density_tolerance",
+                                         "commutator_tolerance", "loose_tolerance",
+                                         "energy_roundoff")],
+        *[(f, ctypes.c_void_p) for f in ("energy", "cmax", "e_old_in", "active_in", "e_old_out",
+                                         "final_e", "final_de", "final_drms", "partial",
+                                         "active_out", "iters", "converged", "flags")],
+        *[(f, ctypes.c_void_p * 2) for f in ("d_new", "c_new", "f", "d", "c", "d_final", "c_final",
+                                             "f_final")],
+    ]
+
+
 # name -> argtypes (every function returns int status unless listed below)
 _P = ctypes.c_void_p
 _SIGNATURES = {
@@ -125,6 +143,7 @@ _SIGNATURES = {
     "vqc_sp2_purify": ([_P, ctypes.c_int32, ctypes.c_int32, ctypes.c_double, ctypes.c_double,
                         ctypes.c_int32, ctypes.c_int32, _P, _P, ctypes.c_uint64, _P, _P],
                        ctypes.c_int),
+    "vqc_scf_record": ([ctypes.POINTER(ScfRecordArgs), _P], ctypes.c_int),
     "vqc_unpack_aux_major": ([_P, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                               ctypes.c_int32, _P, _P], ctypes.c_int),
     "vqc_split_tf32": ([_P, _P, _P, ctypes.c_int64, _P], ctypes.c_int),

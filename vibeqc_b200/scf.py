@@ -666,6 +666,76 @@ def _scf_post(nb, n, x, hist, with_rho, device) -> _SCFPost:
     return p
 
 
+class SCFRecord:
+    """State of a chunk's SCF over its iterations, kept on the device (vqc_scf_record).
+
+    ``d`` and ``c`` are the current density and factor of each spin, ``*_final``
+    those of a molecule's last active iteration; ``step`` tests convergence and
+    moves both on.
+    """
+
+    def __init__(self, ds: list, cs: list, energy_tolerance: float, density_tolerance: float,
+                 commutator_tolerance: float):
+        nb, n, _ = ds[0].shape
+        f64 = dict(dtype=torch.float64, device=ds[0].device)
+        i32 = dict(dtype=torch.int32, device=ds[0].device)
+        self.d = [d.contiguous().clone() for d in ds]
+        self.c = [c.contiguous().clone() for c in cs]
+        self.d_final = [d.clone() for d in ds]
+        self.c_final = [c.clone() for c in cs]
+        self.f_final = [torch.zeros_like(d) for d in self.d]
+        # read and written in turn: every CTA of a molecule reads the old state
+        self._active = torch.ones(2, nb, **i32)
+        self._e_old = torch.full((2, nb), float("nan"), **f64)
+        self.energy = torch.zeros(nb, **f64)
+        self.energy_change = torch.full((nb,), float("inf"), **f64)
+        self.density_rms = torch.full((nb,), float("inf"), **f64)
+        self.iterations = torch.zeros(nb, dtype=torch.int64, device=ds[0].device)
+        self._converged = torch.zeros(nb, **i32)
+        self._flags = torch.zeros(2, **i32)
+        self._partial = torch.empty(nb, 32, **f64)
+        self._now = 0
+        a = self._args = _lib.ScfRecordArgs()
+        a.struct_size = ctypes.sizeof(a)
+        a.nmol, a.n, a.ncol, a.nspin = nb, n, cs[0].shape[2], len(ds)
+        a.energy_tolerance, a.density_tolerance = energy_tolerance, density_tolerance
+        a.commutator_tolerance, a.loose_tolerance = commutator_tolerance, ANCHOR_COMMUTATOR
+        a.energy_roundoff = ENERGY_ROUNDOFF_FACTOR * DOUBLE_EPS
+        a.final_e, a.final_de = self.energy.data_ptr(), self.energy_change.data_ptr()
+        a.final_drms, a.partial = self.density_rms.data_ptr(), self._partial.data_ptr()
+        a.iters, a.converged = self.iterations.data_ptr(), self._converged.data_ptr()
+        a.flags = self._flags.data_ptr()
+        for s in range(len(ds)):
+            a.d[s], a.c[s] = self.d[s].data_ptr(), self.c[s].data_ptr()
+            a.d_final[s], a.c_final[s] = self.d_final[s].data_ptr(), self.c_final[s].data_ptr()
+            a.f_final[s] = self.f_final[s].data_ptr()
+
+    @property
+    def active(self) -> torch.Tensor:
+        return self._active[self._now] != 0
+
+    @property
+    def converged(self) -> torch.Tensor:
+        return self._converged != 0
+
+    def step(self, iteration: int, may_converge: bool, energy, cmax, fs, new_ds, new_cs) -> tuple:
+        """(any molecule still active, any active molecule's residual above ANCHOR_COMMUTATOR)."""
+        keep = [t.contiguous() for t in (energy, cmax, *fs, *new_ds, *new_cs)]
+        a, k = self._args, len(fs)
+        a.iteration, a.may_converge = iteration, int(may_converge)
+        a.energy, a.cmax = keep[0].data_ptr(), keep[1].data_ptr()
+        for s in range(k):
+            a.f[s], a.d_new[s] = keep[2 + s].data_ptr(), keep[2 + k + s].data_ptr()
+            a.c_new[s] = keep[2 + 2 * k + s].data_ptr()
+        old, new = self._now, 1 - self._now
+        a.e_old_in, a.active_in = self._e_old[old].data_ptr(), self._active[old].data_ptr()
+        a.e_old_out, a.active_out = self._e_old[new].data_ptr(), self._active[new].data_ptr()
+        _lib.call("vqc_scf_record", ctypes.byref(a), _stream_ptr())
+        self._now = new
+        active, tight = self._flags.tolist()
+        return bool(active), bool(tight)
+
+
 def run_scf(chunk: Chunk, ints: ChunkIntegrals, xyz: torch.Tensor, *, precision: str = "fp64",
             max_iterations: int = 100, energy_tolerance: float = 1e-10,
             density_tolerance: float = 1e-8, diis_history: int = 8,
@@ -743,18 +813,9 @@ def run_scf(chunk: Chunk, ints: ChunkIntegrals, xyz: torch.Tensor, *, precision:
         f0 = torch.where(warm_used[:, None, None], -0.5 * (s @ wd @ s), h)
     d, co = density_from(f0, guess)
     c = xo @ co  # AO occupied factor, D = 2 C C^T
-    active = torch.ones(nb, dtype=torch.bool, device=dev)
-    e_old = torch.full((nb,), float("nan"), dtype=torch.float64, device=dev)
-    final_e = torch.zeros(nb, dtype=torch.float64, device=dev)
-    final_de = torch.full((nb,), float("inf"), dtype=torch.float64, device=dev)
-    final_drms = torch.full((nb,), float("inf"), dtype=torch.float64, device=dev)
-    iters = torch.zeros(nb, dtype=torch.int64, device=dev)
-    converged = torch.zeros(nb, dtype=torch.bool, device=dev)
-    d_final = d.clone()
-    c_final = c.clone()
-    f_final = torch.zeros_like(d)
+    state = SCFRecord([d], [c], energy_tolerance, density_tolerance, min(1e-8, density_tolerance))
+    d, c = state.d[0], state.c[0]  # advanced in place by state.step
     post = None
-    comm_tol = min(1e-8, density_tolerance)
     # mixed precision runs two phases per chunk:
     #   "tc":     plain tensor-core J/K until max|FDS-SDF| <= ANCHOR_COMMUTATOR
     #             for every active molecule (or MIXED_ITERATION_CAP).  Their
@@ -807,7 +868,6 @@ def run_scf(chunk: Chunk, ints: ChunkIntegrals, xyz: torch.Tensor, *, precision:
                 post.gram.copy_(prev.gram)
                 post.count.copy_(prev.count)
         f, energy, cmax, f_ext = post.run(j, k, d, rho)
-        energy = energy.clone()
         TIMER_ctx.__exit__(None, None, None)
         # the tensor-core phase only needs the projector to its own accuracy
         if phase == "anchor":
@@ -818,40 +878,18 @@ def run_scf(chunk: Chunk, ints: ChunkIntegrals, xyz: torch.Tensor, *, precision:
             d_new, co = density_from(f_ext, co, 1e-11 if phase == "exact" else 1e-8)
         TIMER_ctx = TIMER.stage("scf_other")
         TIMER_ctx.__enter__()
-        c_new = xo @ co
-        de = (energy - e_old).abs()
-        de = torch.where(torch.isnan(de), torch.full_like(de, float("inf")), de)
-        drms = ((d_new - d) ** 2).mean(dim=(1, 2)).sqrt()
-        guard = ENERGY_ROUNDOFF_FACTOR * DOUBLE_EPS * torch.clamp(
-            torch.maximum(energy.abs(), e_old.abs().nan_to_num(0.0)), min=1.0)
-        done = (de < energy_tolerance + guard) & (drms < density_tolerance) & (cmax <= comm_tol)
-        if phase == "tc":
-            loose = cmax <= ANCHOR_COMMUTATOR
-            if bool((loose | ~active).all()) or phase_iterations >= MIXED_ITERATION_CAP:
-                phase, phase_iterations = "anchor", 0
-            done = torch.zeros_like(done)
+        was = None if trace is None else state.active
+        running, tight = state.step(it, phase != "tc", energy, cmax, [f], [d_new], [xo @ co])
+        if phase == "tc" and (not tight or phase_iterations >= MIXED_ITERATION_CAP):
+            phase, phase_iterations = "anchor", 0
         if trace is not None:
-            trace.append((it, phase, float(de[active].max()) if bool(active.any()) else 0.0,
-                          float(cmax[active].max()) if bool(active.any()) else 0.0,
-                          int(active.sum())))
-        newly = done & active
-        # record the state of molecules that are still active
-        final_e = torch.where(active, energy, final_e)
-        final_de = torch.where(active, de, final_de)
-        final_drms = torch.where(active, drms, final_drms)
-        iters = torch.where(active, torch.full_like(iters, it), iters)
-        d_final = torch.where(active[:, None, None], d, d_final)
-        c_final = torch.where(active[:, None, None], c, c_final)
-        f_final = torch.where(active[:, None, None], f, f_final)
-        converged |= newly
-        active &= ~newly
-        e_old = energy
-        if not bool(active.any()):
-            TIMER_ctx.__exit__(None, None, None)
-            break
-        d = torch.where(active[:, None, None], d_new, d)
-        c = torch.where(active[:, None, None], c_new, c)
+            any_was = bool(was.any())
+            trace.append((it, phase, float(state.energy_change[was].max()) if any_was else 0.0,
+                          float(cmax[was].max()) if any_was else 0.0, int(was.sum())))
         TIMER_ctx.__exit__(None, None, None)
+        if not running:
+            break
+    final_e, d_final, c_final = state.energy, state.d_final[0], state.c_final[0]
     if jk.precision == "mixed" and anchored:
         # rho and U = B C at the converged orbitals for the gradient: the
         # anchor's FP64 U0 plus the tensor-core increment
@@ -864,9 +902,10 @@ def run_scf(chunk: Chunk, ints: ChunkIntegrals, xyz: torch.Tensor, *, precision:
     else:
         exact_half = None
     return {
-        "energy": final_e, "converged": converged, "iterations": iters,
-        "energy_change": final_de, "density_rms": final_drms, "density": d_final,
-        "orbitals": c_final, "fock": f_final, "exact_half": exact_half,
+        "energy": final_e, "converged": state.converged, "iterations": state.iterations,
+        "energy_change": state.energy_change, "density_rms": state.density_rms,
+        "density": d_final, "orbitals": c_final, "fock": state.f_final[0],
+        "exact_half": exact_half,
         "mixed_iterations": mixed_iterations, "anchors": anchors,
         "warm_used": warm_used, "warm_fallback": warm_fallback,
         "metric": mf, "orthogonalizer": xo, "enuc": enuc, "charges": zs, "jk": jk,

@@ -256,18 +256,10 @@ def run_scf_uhf(chunk, ints, xyz: torch.Tensor, *, precision: str = "fp64",
         return [_pad_columns(xo @ c_, width) * INV_SQRT2 for c_ in cos_]
 
     cs = channel_factors(cos)
-    active = torch.ones(nb, dtype=torch.bool, device=dev)
-    e_old = torch.full((nb,), float("nan"), dtype=torch.float64, device=dev)
-    final_e = torch.zeros(nb, dtype=torch.float64, device=dev)
-    final_de = torch.full((nb,), float("inf"), dtype=torch.float64, device=dev)
-    final_drms = torch.full((nb,), float("inf"), dtype=torch.float64, device=dev)
-    iters = torch.zeros(nb, dtype=torch.int64, device=dev)
-    converged = torch.zeros(nb, dtype=torch.bool, device=dev)
-    d_final = [d_.clone() for d_ in ds]
-    c_final = [c_.clone() for c_ in cs]
-    f_final = [torch.zeros_like(h), torch.zeros_like(h)]
+    state = scfm.SCFRecord(ds, cs, energy_tolerance, density_tolerance,
+                           min(1e-8, density_tolerance))
+    ds, cs = state.d, state.c  # advanced in place by state.step
     post = None
-    comm_tol = min(1e-8, density_tolerance)
     phase = "tc" if jk.precision == "mixed" else "exact"
     phase_iterations = 0
     mixed_iterations = 0
@@ -317,8 +309,6 @@ def run_scf_uhf(chunk, ints, xyz: torch.Tensor, *, precision: str = "fp64",
                 post.gram.copy_(prev.gram)
                 post.count.copy_(prev.count)
         f, energy, cmax, f_ext = post.run(j, ka, kb, ds[0], ds[1], rho)
-        energy = energy.clone()
-        f = f.clone()
         ctx.__exit__(None, None, None)
         new_d, new_co = [], []
         for sp in range(2):
@@ -333,40 +323,15 @@ def run_scf_uhf(chunk, ints, xyz: torch.Tensor, *, precision: str = "fp64",
             new_co.append(co_)
         ctx = TIMER.stage("scf_other")
         ctx.__enter__()
-        new_c = channel_factors(new_co)
-        de = (energy - e_old).abs()
-        de = torch.where(torch.isnan(de), torch.full_like(de, float("inf")), de)
-        drms = ((((new_d[0] - ds[0]) ** 2).sum(dim=(1, 2)) + ((new_d[1] - ds[1]) ** 2).sum(dim=(1, 2)))
-                / (2 * n * n)).sqrt()
-        guard = scfm.ENERGY_ROUNDOFF_FACTOR * scfm.DOUBLE_EPS * torch.clamp(
-            torch.maximum(energy.abs(), e_old.abs().nan_to_num(0.0)), min=1.0)
-        done = (de < energy_tolerance + guard) & (drms < density_tolerance) & (cmax <= comm_tol)
-        if phase == "tc":
-            loose = cmax <= scfm.ANCHOR_COMMUTATOR
-            if bool((loose | ~active).all()) or phase_iterations >= scfm.MIXED_ITERATION_CAP:
-                phase, phase_iterations = "anchor", 0
-            done = torch.zeros_like(done)
-        newly = done & active
-        final_e = torch.where(active, energy, final_e)
-        final_de = torch.where(active, de, final_de)
-        final_drms = torch.where(active, drms, final_drms)
-        iters = torch.where(active, torch.full_like(iters, it), iters)
-        keep = active[:, None, None]
-        for sp in range(2):
-            d_final[sp] = torch.where(keep, ds[sp], d_final[sp])
-            c_final[sp] = torch.where(keep, cs[sp], c_final[sp])
-            f_final[sp] = torch.where(keep, f[sp], f_final[sp])
-        converged |= newly
-        active &= ~newly
-        e_old = energy
-        if not bool(active.any()):
-            ctx.__exit__(None, None, None)
-            break
-        for sp in range(2):
-            ds[sp] = torch.where(keep & active[:, None, None], new_d[sp], ds[sp])
-            cs[sp] = torch.where(keep & active[:, None, None], new_c[sp], cs[sp])
-            cos[sp] = new_co[sp]
+        running, tight = state.step(it, phase != "tc", energy, cmax, [f[0], f[1]], new_d,
+                                    channel_factors(new_co))
+        if phase == "tc" and (not tight or phase_iterations >= scfm.MIXED_ITERATION_CAP):
+            phase, phase_iterations = "anchor", 0
         ctx.__exit__(None, None, None)
+        if not running:
+            break
+        cos = new_co
+    final_e, d_final, c_final = state.energy, state.d_final, state.c_final
     if jk.precision == "mixed" and anchored:
         exact_half = [jk.anchored_half(c_final[sp], sp) for sp in range(2)]
         jk.release_tensor_core_buffers()
@@ -375,10 +340,10 @@ def run_scf_uhf(chunk, ints, xyz: torch.Tensor, *, precision: str = "fp64",
     else:
         exact_half = None
     return {
-        "energy": final_e, "converged": converged, "iterations": iters,
-        "energy_change": final_de, "density_rms": final_drms,
+        "energy": final_e, "converged": state.converged, "iterations": state.iterations,
+        "energy_change": state.energy_change, "density_rms": state.density_rms,
         "density": d_final[0] + d_final[1], "spin_densities": d_final,
-        "orbitals": c_final, "fock": f_final, "exact_half": exact_half,
+        "orbitals": c_final, "fock": state.f_final, "exact_half": exact_half,
         "mixed_iterations": mixed_iterations, "anchors": anchors,
         "warm_used": warm_used, "warm_fallback": warm_fallback,
         "metric": mf, "orthogonalizer": xo, "enuc": enuc, "charges": zs, "jk": jk,
