@@ -182,19 +182,21 @@ struct Triple {
 };
 
 // Class-molecule entry of a CTA: the last whose chunk_begin is not above the
-// block index.  Warps look at 32 entries per load instead of bisecting, whose
-// dependent loads every CTA would wait for.  Every lane of a full warp must
-// call it.
+// block index.  A warp looks at 32 evenly spaced entries of the remaining range
+// per load, so n entries take log32(n) dependent loads, which every CTA waits
+// for: one up to 32 molecules, three up to 32768 (a bisection takes 5 and 15).
+// Every lane of a full warp must call it.
 __device__ __forceinline__ int find_cm(const ClassMol* __restrict__ cms, int ncm, int block) {
   const int lane = threadIdx.x & 31;
-  int n = 0;
-  for (int i = 0; i < ncm; i += 32) {
-    const bool below = i + lane < ncm && cms[i + lane].chunk_begin <= block;
-    const int hits = __popc(__ballot_sync(0xffffffffu, below));
-    n += hits;
-    if (hits < 32) break;
+  int lo = 0, n = ncm;  // the entry lies in [lo, lo + n), and cms[lo] is not above
+  for (;;) {
+    const int step = (n + 31) / 32, i = lane * step;
+    const bool below = i < n && cms[lo + i].chunk_begin <= block;
+    const int skip = (__popc(__ballot_sync(0xffffffffu, below)) - 1) * step;
+    lo += skip;
+    if (step == 1) return lo;
+    n = min(step, n - skip);
   }
-  return n - 1;
 }
 
 // One-electron kernels: k1eLanes lanes per shell pair.  With one thread per
