@@ -235,7 +235,7 @@ int Plan::build(const vqc_batch_desc& d) {
         if (pcnt[c][m]) one.push_back(ClassMol{m, pbeg[c][m], 0, 0, pcnt[c][m], 0});
       int nab = 1;
       for (const int2& pr : pl[c]) nab = std::max(nab, orb_h.nprim[pr.x] * orb_h.nprim[pr.y]);
-      if ((st = add_class(cls1e, la, lb, 0, dpairs[c], one, 128))) return st;
+      if ((st = add_class(cls1e, la, lb, 0, dpairs[c], one, k1ePairs))) return st;
       for (int lc = 0; lc <= kMaxKernelL; ++lc) {
         std::vector<ClassMol> cm3;
         for (int m = 0; m < nmol; ++m) {

@@ -541,10 +541,8 @@ __global__ void __launch_bounds__(128)
   __shared__ AtomSums sums;
   for (int i = threadIdx.x; i < 3 * kAccAtoms; i += blockDim.x) sums.v[i] = 0.0;
   __syncthreads();
-  const int chunk = blockIdx.x / k1eLanes;
-  const ClassMol cm = cms[find_cm(cms, ncm, chunk)];
-  const int t = (chunk - cm.chunk_begin) * 128 +
-                ((blockIdx.x % k1eLanes) * 128 + threadIdx.x) / k1eLanes;
+  const ClassMol cm = cms[find_cm(cms, ncm, blockIdx.x)];
+  const int t = (blockIdx.x - cm.chunk_begin) * k1ePairs + threadIdx.x / k1eLanes;
   const bool valid = t < cm.ntriples;
   const DevMol mol = mols[cm.mol];
   const bool local = mol.natom <= kAccAtoms;
@@ -735,8 +733,8 @@ static void glaunch2(const ClassLaunch& cl, const KernelArgs& k, cudaStream_t st
 
 template <int LA, int LB, bool SPH>
 static void glaunch1(const ClassLaunch& cl, const KernelArgs& k, cudaStream_t st) {
-  grad1e_kernel<LA, LB, SPH><<<cl.nblocks * k1eLanes, 128, 0, st>>>(k.orb, k.xyz, k.charge, k.mols, cl.pairs,
-                                                          cl.cms, cl.ncm, k.w1, k.w2, k.grad);
+  grad1e_kernel<LA, LB, SPH><<<cl.nblocks, 128, 0, st>>>(k.orb, k.xyz, k.charge, k.mols, cl.pairs, cl.cms,
+                                                         cl.ncm, k.w1, k.w2, k.grad);
 }
 
 #define VQC_G3(LA, LB, LC)                                              \

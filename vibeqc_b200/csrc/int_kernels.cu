@@ -446,10 +446,8 @@ __global__ void __launch_bounds__(128)
   constexpr int MODE = SPH ? 0 : 1;
   constexpr Cart<LA> ca{};
   constexpr Cart<LB> cb{};
-  const int chunk = blockIdx.x / k1eLanes;
-  const ClassMol cm = cms[find_cm(cms, ncm, chunk)];
-  const int t = (chunk - cm.chunk_begin) * 128 +
-                ((blockIdx.x % k1eLanes) * 128 + threadIdx.x) / k1eLanes;
+  const ClassMol cm = cms[find_cm(cms, ncm, blockIdx.x)];
+  const int t = (blockIdx.x - cm.chunk_begin) * k1ePairs + threadIdx.x / k1eLanes;
   const bool valid = t < cm.ntriples;
   const DevMol mol = mols[cm.mol];
   const Lanes1e ln(mol.natom);
@@ -587,8 +585,8 @@ static void launch2(const ClassLaunch& cl, const KernelArgs& k, cudaStream_t st)
 
 template <int LA, int LB, bool SPH>
 static void launch1(const ClassLaunch& cl, const KernelArgs& k, cudaStream_t st) {
-  int1e_kernel<LA, LB, SPH><<<cl.nblocks * k1eLanes, 128, 0, st>>>(k.orb, k.xyz, k.charge, k.mols, cl.pairs,
-                                                        cl.cms, cl.ncm, k.out, k.out2, k.out3);
+  int1e_kernel<LA, LB, SPH><<<cl.nblocks, 128, 0, st>>>(k.orb, k.xyz, k.charge, k.mols, cl.pairs, cl.cms,
+                                                        cl.ncm, k.out, k.out2, k.out3);
 }
 
 #define VQC_L3(LA, LB, LC)                                              \

@@ -205,7 +205,11 @@ __device__ __forceinline__ int find_cm(const ClassMol* __restrict__ cms, int ncm
 // FP64 pipe 4 % active).  The lanes split the nuclei; with fewer nuclei than
 // lanes, the primitive pairs as well.  (ss) derivatives of 12 x (H2O)6 0.290 ->
 // 0.068 ms, (ps) 0.245 -> 0.082; (ss) values of 8 x (H2O)9 0.151 -> 0.056.
+// A CTA takes k1ePairs pairs of one molecule.  A CTA of 128 pairs spread over
+// eight launched ones left most of these empty for small molecules: 16384
+// waters 6.4 -> 2.2 ms, 32768 H2 0.58 -> 0.14 (one lane a pair 2.2 and 0.22).
 constexpr int k1eLanes = 8;
+constexpr int k1ePairs = 128 / k1eLanes;
 struct Lanes1e {
   int lane, c0, dc, k0, dk;
   __device__ __forceinline__ explicit Lanes1e(int natom) {
