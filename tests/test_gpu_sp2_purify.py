@@ -64,3 +64,34 @@ def test_layouts_and_arguments():
     assert (purify_sp2(strided, 9) - want).abs().max().item() < 2e-11
     with pytest.raises(_lib.VqcError):
         _purify_fp64(_fock(1, 113, 9, 1)[0], 9, 96, 1e-11, 1)
+
+
+@pytest.mark.parametrize("path,nb,n", [(2, 1, 512), (0, 1, 1000), (3, 1, 1400), (0, 2, 700)])
+def test_groups_of_many_tiles(path, nb, n):
+    """More tiles than the 128 CTAs a group once had, up to every resident CTA."""
+    f, want = _fock(nb, n, n // 5, n)
+    got = _purify_fp64(f, n // 5, 96, 1e-11, path)
+    assert (got - want).abs().max().item() < 4e-11  # n eps |F| / gap, as above, at n = 1400
+    assert torch.equal(got, got.transpose(1, 2))
+
+
+@pytest.mark.parametrize("n", [512, 1000])
+def test_one_large_molecule_uses_every_cta(n):
+    """About 50 squarings with their updates: less than the time of 75 library squarings.
+
+    Groups of at most 128 CTAs took 108 (n = 512) and 99 (n = 1000) of them, every CTA 62 and 39.
+    """
+    f, _ = _fock(1, n, n // 5, n)
+    times = []
+    for call in (lambda: _purify_fp64(f, n // 5, 96, 1e-11),
+                 lambda: [torch.bmm(f, f) for _ in range(75)]):
+        best = float("inf")
+        for _ in range(5):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            call()
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        times.append(best)
+    assert times[0] < times[1], times

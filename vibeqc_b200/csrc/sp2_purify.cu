@@ -206,7 +206,6 @@ __global__ void __launch_bounds__(kSmallThreads)
 constexpr int kKB = 32;          // K columns per pipeline stage
 constexpr int kLdS = kKB + 4;    // stage row stride (4 modulo 16 doubles)
 constexpr int kStages = 3;
-constexpr int kMaxGroup = 128;   // CTAs per group (one partial-sum slot per thread)
 constexpr unsigned long long kWaitNs = 2000000000ull;
 
 struct GroupParams {
@@ -458,7 +457,6 @@ static Choice plan_groups(int nmol, int n, int bm, int resident, int sms, double
     const int groups = (nmol + r - 1) / r;
     int g = resident / groups;
     g = g > tiles ? tiles : g;
-    g = g > kMaxGroup ? kMaxGroup : g;
     const int per = (tiles + g - 1) / g;
     g = (tiles + per - 1) / per;  // no CTA without a tile in the last pass
     const int share = (groups * g + sms - 1) / sms;
