@@ -48,3 +48,34 @@ def test_unpack_aux_major(nb, n, x, ld):
     full = bp[:, hi * (hi + 1) // 2 + lo]  # (nb, mu, nu, Q)
     assert torch.equal(b[..., :n], full.transpose(2, 3).float())
     assert (b[..., n:] == 0).all()
+
+
+@pytest.mark.parametrize("x,ldq", [(92, 92), (94, 96), (96, 96), (128, 128), (254, 256), (256, 256),
+                                   (258, 260), (510, 512)])
+def test_anchor_combine_column_groups(x, ldq):
+    """Either side of the rule (96 columns) and of the 128-column groups, taken two at a time."""
+    test_anchor_combine(300, x, ldq, 0)
+
+
+def _time(call):
+    best = float("inf")
+    for _ in range(8):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        call()
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b))
+    return best
+
+
+def test_rate_of_the_combination_in_place():
+    """Mode 1 moves as much as mode 0, so it takes no more than 1.2 of its time (1.26 with one group at a time)."""
+    rows, x = 100 * 32 * 20, 500
+    u0 = torch.zeros(rows, x, device="cuda", dtype=torch.float64)
+    dh, dl, vh, vl = (torch.zeros(rows, x, device="cuda") for _ in range(4))
+    st = torch.cuda.current_stream().cuda_stream
+    times = [_time(lambda: _lib.call("vqc_anchor_combine", u0.data_ptr(), dh.data_ptr(), dl.data_ptr(),
+                                     vh.data_ptr(), vl.data_ptr(), rows, x, x, 1.0, mode, st))
+             for mode in (0, 1)]
+    assert times[1] < 1.2 * times[0], times

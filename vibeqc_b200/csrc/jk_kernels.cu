@@ -227,7 +227,13 @@ __device__ __forceinline__ void split_rna(float v, float& h, float& l) {
 // element kernel below spends a 64-bit division on each).  HBM-bound: 24 bytes
 // per element read and written once.  Needs ldq % 4 == 0, 16-byte aligned
 // arrays and, for the pairs of U0, even x.
-// 10 x (H2O)11: 0.949 -> 0.838 ms (4.4 GB; 81 % of the measured copy rate).
+// Element kernel -> this one, mode 0 / mode 1: 4 x (N = 384, X = 1856) 1.18 ->
+// 0.83 / 1.09 -> 0.91 ms, 256 x (48, 232) 0.150 -> 0.108 / 0.141 -> 0.112,
+// 10 x (H2O)11 0.955 -> 0.716 / 0.888 -> 0.764 (4.4 GB; 94 % / 88 % of the
+// measured copy rate).
+// Shorter rows leave most lanes idle: 65536 rows of 64 columns, mode 1 from L2,
+// 18.6 us against 14.5; from 96 columns on it is never behind.
+constexpr int kCombine4Columns = 96;
 template <int MODE>
 __global__ void __launch_bounds__(256)
     anchor_combine4_kernel(double* __restrict__ u0, const float* __restrict__ du_hi,
@@ -238,34 +244,47 @@ __global__ void __launch_bounds__(256)
        r += (long long)gridDim.x * 8) {
     double* u = u0 + r * x;
     const long long e0 = r * ldq;
-#pragma unroll 2
-    for (int q = 4 * lane; q < ldq; q += 128) {
-      const float4 h = __ldcs(reinterpret_cast<const float4*>(du_hi + e0 + q));
-      const float4 l = __ldcs(reinterpret_cast<const float4*>(du_lo + e0 + q));
-      // x is even: a pair is inside the row or outside it
-      const bool in0 = q < x, in1 = q + 2 < x;
-      const double2 z = make_double2(0.0, 0.0);
-      double2 a = in0 ? *reinterpret_cast<const double2*>(u + q) : z;
-      double2 b = in1 ? *reinterpret_cast<const double2*>(u + q + 2) : z;
-      a.x += alpha * ((double)h.x + (double)l.x);
-      a.y += alpha * ((double)h.y + (double)l.y);
-      b.x += alpha * ((double)h.z + (double)l.z);
-      b.y += alpha * ((double)h.w + (double)l.w);
-      if constexpr (MODE == 1) {
-        if (in0) *reinterpret_cast<double2*>(u + q) = a;
-        if (in1) *reinterpret_cast<double2*>(u + q + 2) = b;
-      } else {
-        float4 vh = make_float4(0.0f, 0.0f, 0.0f, 0.0f), vl = vh;
-        if (in0) {
-          split_rna((float)a.x, vh.x, vl.x);
-          split_rna((float)a.y, vh.y, vl.y);
+    // two groups of columns at a time: in mode 1 the loads of the second would
+    // else wait for the stores of the first
+    for (int q0 = 4 * lane; q0 < ldq; q0 += 256) {
+      float4 h[2], l[2];
+      double2 a[2], b[2];
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        const int q = q0 + 128 * g;
+        if (q >= ldq) break;
+        h[g] = __ldcs(reinterpret_cast<const float4*>(du_hi + e0 + q));
+        l[g] = __ldcs(reinterpret_cast<const float4*>(du_lo + e0 + q));
+        // x is even: a pair is inside the row or outside it
+        const double2 z = make_double2(0.0, 0.0);
+        a[g] = q < x ? *reinterpret_cast<const double2*>(u + q) : z;
+        b[g] = q + 2 < x ? *reinterpret_cast<const double2*>(u + q + 2) : z;
+      }
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        const int q = q0 + 128 * g;
+        if (q >= ldq) break;
+        const bool in0 = q < x, in1 = q + 2 < x;
+        a[g].x += alpha * ((double)h[g].x + (double)l[g].x);
+        a[g].y += alpha * ((double)h[g].y + (double)l[g].y);
+        b[g].x += alpha * ((double)h[g].z + (double)l[g].z);
+        b[g].y += alpha * ((double)h[g].w + (double)l[g].w);
+        if constexpr (MODE == 1) {
+          if (in0) *reinterpret_cast<double2*>(u + q) = a[g];
+          if (in1) *reinterpret_cast<double2*>(u + q + 2) = b[g];
+        } else {
+          float4 vh = make_float4(0.0f, 0.0f, 0.0f, 0.0f), vl = vh;
+          if (in0) {
+            split_rna((float)a[g].x, vh.x, vl.x);
+            split_rna((float)a[g].y, vh.y, vl.y);
+          }
+          if (in1) {
+            split_rna((float)b[g].x, vh.z, vl.z);
+            split_rna((float)b[g].y, vh.w, vl.w);
+          }
+          *reinterpret_cast<float4*>(v_hi + e0 + q) = vh;
+          *reinterpret_cast<float4*>(v_lo + e0 + q) = vl;
         }
-        if (in1) {
-          split_rna((float)b.x, vh.z, vl.z);
-          split_rna((float)b.y, vh.w, vl.w);
-        }
-        *reinterpret_cast<float4*>(v_hi + e0 + q) = vh;
-        *reinterpret_cast<float4*>(v_lo + e0 + q) = vl;
       }
     }
   }
@@ -311,7 +330,7 @@ extern "C" int vqc_anchor_combine(double* u0, const float* du_hi, const float* d
   // four columns a lane where the rows allow it, else element by element
   const uintptr_t all = (uintptr_t)u0 | (uintptr_t)du_hi | (uintptr_t)du_lo |
                         (mode == 0 ? (uintptr_t)v_hi | (uintptr_t)v_lo : 0);
-  if (x % 2 == 0 && ld_aux % 4 == 0 && all % 16 == 0) {
+  if (x % 2 == 0 && ld_aux % 4 == 0 && ld_aux >= kCombine4Columns && all % 16 == 0) {
     const long long want = (rows + 7) / 8;
     const int grid = (int)(want > 16 * 148 ? 16 * 148 : want);
     if (mode == 0)
