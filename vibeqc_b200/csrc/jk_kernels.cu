@@ -177,8 +177,14 @@ __global__ void __launch_bounds__(256)
 // bp[mol][(max(mu,nu)(max+1)/2 + min)][Q] (FP64); padding columns are zeroed.
 // A transpose per mu, bound by HBM: 32 x 32 tiles through shared memory, so
 // that warps read 256 bytes along Q and write 128 along nu (without the tile a
-// warp read 8 bytes from each of 32 rows). 
+// warp reads 8 bytes from each of 32 rows).  Against the element kernel below:
+// 4 x (N = 384, X = 1856) 9.3 -> 3.4 ms, 8 x (216, 1044) 1.54 -> 1.24,
+// 2048 x (24, 116) 0.60 -> 0.52.
 constexpr int kUnpackTile = 32;
+// Rows up to this long leave half of a tile or more empty: element by element,
+// 8192 x (7, 113) 0.24 ms (tiles 0.46), 1024 x (16, 116) 0.143 (0.154); the
+// tiles are ahead from 20 on (0.208 against 0.222).
+constexpr int kUnpackShortRow = 16;
 __global__ void __launch_bounds__(256)
     unpack_aux_major_kernel(const double* __restrict__ bp, int n, int x, int ld,
                             float* __restrict__ b) {
@@ -206,6 +212,24 @@ __global__ void __launch_bounds__(256)
       if (q < x && nu < ld) dst[(size_t)q * ld + nu] = tile[lane][r];
     }
     __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(256)
+    unpack_short_rows_kernel(const double* __restrict__ bp, int n, int x, int ld, float* __restrict__ b) {
+  const int mol = blockIdx.z, mu = blockIdx.y;
+  const size_t p = (size_t)n * (n + 1) / 2;
+  const double* src = bp + (size_t)mol * p * x;
+  float* dst = b + ((size_t)mol * n + mu) * (size_t)x * ld;
+  const size_t total = (size_t)x * ld;
+  for (size_t e = (size_t)blockIdx.x * 256 + threadIdx.x; e < total; e += (size_t)gridDim.x * 256) {
+    const int q = (int)(e / ld), nu = (int)(e % ld);
+    float v = 0.0f;
+    if (nu < n) {
+      const size_t hi = mu > nu ? mu : nu, lo = mu > nu ? nu : mu;
+      v = (float)src[(hi * (hi + 1) / 2 + lo) * x + q];
+    }
+    dst[e] = v;
   }
 }
 
@@ -454,6 +478,13 @@ extern "C" int vqc_unpack_aux_major(const double* b_packed, int32_t nmol, int32_
   if (!b_packed || !b_aux_major || nmol <= 0 || nao <= 0 || naux <= 0 || ld_ao < nao ||
       nmol > 65535 || nao > 65535)
     return fail(VQC_STATUS_INVALID_ARGUMENT, "unpack_aux_major: bad argument");
+  if (ld_ao <= kUnpackShortRow) {
+    const size_t ctas = ((size_t)naux * ld_ao + 255) / 256;
+    unpack_short_rows_kernel<<<dim3((int)(ctas > 64 ? 64 : ctas), nao, nmol), 256, 0, (cudaStream_t)stream>>>(
+        b_packed, nao, naux, ld_ao, b_aux_major);
+    count_launch();
+    return cuda_status(cudaGetLastError(), "unpack_aux_major");
+  }
   const size_t tiles = ((size_t)naux + kUnpackTile - 1) / kUnpackTile *
                        (((size_t)ld_ao + kUnpackTile - 1) / kUnpackTile);
   if (tiles > 0x7fffffff) return fail(VQC_STATUS_INVALID_ARGUMENT, "unpack_aux_major: too many tiles");
