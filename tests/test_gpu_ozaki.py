@@ -93,6 +93,46 @@ def test_slices_and_products_match_numpy_restatement_bit_for_bit(ns, upper):
         assert (np.abs(c[z] - exact) <= 2.0 ** (-7 * ns + 1) * k * bound).all()
 
 
+@pytest.mark.parametrize("ns", range(1, 8))
+@pytest.mark.parametrize("k", [112, 113])
+def test_slices_of_every_count(ns, k):
+    """Vector (even columns) and element form, with zero and subnormal rows and digits at the clamp."""
+    rng = np.random.default_rng(100 * ns + k)
+    a = rng.standard_normal((2, 37, k)) * 10.0 ** rng.uniform(-300, 300, size=(2, 37, 1))
+    a[:, 3] = 0.0
+    a[:, 4, 5] = np.ldexp(1.0 - 2.0**-53, 8) * np.abs(a[:, 4]).max()  # its first digit rounds to 128
+    a[0, 5] = 5e-324  # its scale overflows: every digit is at the clamp
+    _, sa_gpu, ea_gpu = _gpu(a, a[:, :16], ns)
+    for z in range(2):
+        with np.errstate(over="ignore"):
+            sa, ea = _np_slices(a[z], ns)
+        assert (ea_gpu[z] == ea).all()
+        for s in range(ns):
+            assert (sa_gpu[z, s] == sa[s]).all()
+
+
+def test_rate_of_fewer_slices():
+    """5 slices write less than 7: no more than 1.1 times their time (1.5 with a run-time count)."""
+    nb, p, x = 8192, 28, 113
+    a = torch.randn(nb, p, x, dtype=torch.float64, device="cuda")
+    sl = torch.empty(nb * 7 * p * 128, dtype=torch.int8, device="cuda")
+    ex = torch.empty(nb * p, dtype=torch.int32, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    times = []
+    for ns in (7, 5):
+        best = float("inf")
+        for _ in range(8):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            _lib.call("vqc_ozaki_slice_rows", a.data_ptr(), nb, p, x, x, p * x, None, ns, sl.data_ptr(), 128,
+                      ex.data_ptr(), st)
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        times.append(best)
+    assert times[1] < 1.1 * times[0], times
+
+
 def test_tensor_core_whitening_matches_fp64_whitening():
     from vibeqc_b200.scf import (Chunk, compute_integrals, factor_metric, whiten_in_place,
                                  whiten_tensor_cores)

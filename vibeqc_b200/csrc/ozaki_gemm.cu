@@ -465,20 +465,18 @@ __device__ __forceinline__ void slice_digits_clamped(double y, int ns, int (&dig
 // leaves it in the low word of the sum.  Only an element whose digit reaches
 // +-128 (|y| within 2^-8 of 1, at most a few per row) needs the clamped form.
 template <int NS>
-__device__ __forceinline__ void slice_digits(double y0, int ns, int (&dig)[kMaxSlices]) {
+__device__ __forceinline__ void slice_digits(double y0, int (&dig)[kMaxSlices]) {
   constexpr double kMagic = 6755399441055744.0;
   double y = y0;
   bool over = false;
 #pragma unroll
-  for (int s = 0; s < kMaxSlices; ++s) {
-    if (s < (NS ? NS : ns)) {
-      const double t = fma(y, 128.0, kMagic);
-      y = fma(y, 128.0, kMagic - t);
-      dig[s] = __double2loint(t);
-      over |= dig[s] > 127 || dig[s] < -127;
-    }
+  for (int s = 0; s < NS; ++s) {
+    const double t = fma(y, 128.0, kMagic);
+    y = fma(y, 128.0, kMagic - t);
+    dig[s] = __double2loint(t);
+    over |= dig[s] > 127 || dig[s] < -127;
   }
-  if (over) slice_digits_clamped(y0, ns, dig);
+  if (over) slice_digits_clamped(y0, NS, dig);
 }
 
 // rows of src (FP64, optionally times a per-column power-of-two scale) ->
@@ -491,10 +489,12 @@ __device__ __forceinline__ void slice_digits(double y0, int ns, int (&dig)[kMaxS
 // 8 x (H2O)10: 2.65 -> 1.39 ms, 2.9 TB/s; the 21 FP64 operations an element
 // takes are next.
 // VEC: 16-byte aligned source and scale rows and 4-byte aligned slice rows.
+// NS: the slice count; a count known only at run time costs the digit loop its
+// unrolling (8192 x (28 rows of 113), 5 slices: 0.34 ms, the earlier form 0.26).
 template <bool VEC, int NS>
 __global__ void __launch_bounds__(256)
     slice_rows_kernel(const double* __restrict__ src, int nmol, long long rows, int cols, long long ld,
-                      long long mol_stride, const double* __restrict__ col_scale, int ns,
+                      long long mol_stride, const double* __restrict__ col_scale,
                       int8_t* __restrict__ dst, int ldd, int* __restrict__ exps) {
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(256)
       if (mx > 0.0) frexp(mx, &e);
     }
     const double inv = ldexp(1.0, -e);
-    int8_t* d = dst + (z * ns * rows + r) * (long long)ldd;
+    int8_t* d = dst + (z * NS * rows + r) * (long long)ldd;
     const long long sstride = rows * (long long)ldd;
     for (int c = 4 * lane; c < cols; c += 128) {
       double v[4];
@@ -547,21 +547,20 @@ __global__ void __launch_bounds__(256)
       int dig[4][kMaxSlices];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        if (odd) slice_digits_clamped(v[k] * inv, ns, dig[k]);
-        else slice_digits<NS>(v[k] * inv, ns, dig[k]);
+        if (odd) slice_digits_clamped(v[k] * inv, NS, dig[k]);
+        else slice_digits<NS>(v[k] * inv, dig[k]);
       }
       if (VEC && c + 4 <= cols) {
 #pragma unroll
-        for (int s = 0; s < kMaxSlices; ++s)
-          if (s < (NS ? NS : ns))
-            *reinterpret_cast<char4*>(d + s * sstride + c) =
-                make_char4((char)dig[0][s], (char)dig[1][s], (char)dig[2][s], (char)dig[3][s]);
+        for (int s = 0; s < NS; ++s)
+          *reinterpret_cast<char4*>(d + s * sstride + c) =
+              make_char4((char)dig[0][s], (char)dig[1][s], (char)dig[2][s], (char)dig[3][s]);
       } else {
 #pragma unroll
-        for (int s = 0; s < kMaxSlices; ++s)
+        for (int s = 0; s < NS; ++s)
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            if (s < (NS ? NS : ns) && c + k < cols) d[s * sstride + c + k] = (int8_t)dig[k][s];
+            if (c + k < cols) d[s * sstride + c + k] = (int8_t)dig[k][s];
       }
     }
     if (lane == 0) exps[z * rows + r] = e;
@@ -603,11 +602,18 @@ extern "C" int vqc_ozaki_slice_rows(const double* src, int32_t nmol, int64_t row
   const bool vec = reinterpret_cast<uintptr_t>(src) % 16 == 0 && ld % 2 == 0 && mol_stride % 2 == 0 &&
                    reinterpret_cast<uintptr_t>(dst) % 4 == 0 && ldd % 4 == 0 &&
                    (!col_scale || (reinterpret_cast<uintptr_t>(col_scale) % 16 == 0 && cols % 2 == 0));
-  auto kern = nslices == oz::kMaxSlices
-                  ? (vec ? oz::slice_rows_kernel<true, oz::kMaxSlices> : oz::slice_rows_kernel<false, oz::kMaxSlices>)
-                  : (vec ? oz::slice_rows_kernel<true, 0> : oz::slice_rows_kernel<false, 0>);
-  kern<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(src, nmol, rows, cols, ld, mol_stride,
-                                                           col_scale, nslices, dst, ldd, exps);
+  static_assert(oz::kMaxSlices == 7, "one kernel per slice count");
+  auto* kern = vec ? oz::slice_rows_kernel<true, 7> : oz::slice_rows_kernel<false, 7>;
+  switch (nslices) {
+    case 1: kern = vec ? oz::slice_rows_kernel<true, 1> : oz::slice_rows_kernel<false, 1>; break;
+    case 2: kern = vec ? oz::slice_rows_kernel<true, 2> : oz::slice_rows_kernel<false, 2>; break;
+    case 3: kern = vec ? oz::slice_rows_kernel<true, 3> : oz::slice_rows_kernel<false, 3>; break;
+    case 4: kern = vec ? oz::slice_rows_kernel<true, 4> : oz::slice_rows_kernel<false, 4>; break;
+    case 5: kern = vec ? oz::slice_rows_kernel<true, 5> : oz::slice_rows_kernel<false, 5>; break;
+    case 6: kern = vec ? oz::slice_rows_kernel<true, 6> : oz::slice_rows_kernel<false, 6>; break;
+  }
+  kern<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(src, nmol, rows, cols, ld, mol_stride, col_scale,
+                                                           dst, ldd, exps);
   count_launch();
   return cuda_status(cudaGetLastError(), "ozaki_slice_rows");
 }
