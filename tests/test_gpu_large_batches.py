@@ -4,11 +4,13 @@ The launch tables hold one entry per molecule and class, which every CTA looks
 up; batches sit at the edges of that search (32 entries per step).
 """
 
+import threading
+
 import numpy as np
 import pytest
 import torch
 
-from vibeqc_b200 import _lib
+from vibeqc_b200 import _lib, geometry
 from vibeqc_b200.plan import NativePlan, make_molecule
 
 pytestmark = pytest.mark.gpu
@@ -112,3 +114,169 @@ def test_cost_of_small_molecules():
     three = _time(lambda: _lib.call("vqc_int3c", plan.handle, xyz.data_ptr(), a.data_ptr(), _stream()))
     assert times[1] < 16 * times[0], times
     assert times[1] < 0.5 * three, (times, three)
+
+
+def _own_plan_gradients(mol, parts, layout):
+    """The contractions of one molecule by itself, with its slices of a batch's weights."""
+    dens, wdens, mbar, abar = parts
+    mat, _, _, met, three = _parts(layout)
+    plan = NativePlan([mol], True)
+    out = _gradients(plan, dens[mat].clone(), wdens[mat].clone(), mbar[met].clone(), abar[three].clone())
+    plan.close()
+    return out
+
+
+def _check_batch(mols, indices):
+    plan = NativePlan(mols, True)
+    weights = _weights(plan, len(mols))
+    got = _gradients(plan, *weights)
+    for i in indices:
+        lay = plan.layout[i]
+        own = _own_plan_gradients(mols[i], weights, lay)
+        for g, want in zip(got, own):
+            # sums of the same terms in another order: some thousand roundings
+            part = g[lay.atom_offset:lay.atom_offset + lay.natom]
+            assert (part - want).abs().max().item() <= 1e-12 * (1.0 + want.abs().max().item())
+    plan.close()
+
+
+@pytest.mark.parametrize("count", [1, 32, 33, 1025, 4500])
+def test_derivatives_do_not_depend_on_the_batch(count):
+    """Molecules of a few chunks: sums straight to global memory."""
+    kinds = _molecules()
+    step = max(1, count // 23)
+    _check_batch([kinds[i % len(kinds)] for i in range(count)],
+                 sorted({*range(0, count, step), count - 1}))
+
+
+@pytest.mark.parametrize("waters,count", [(4, 40), (6, 13)])
+def test_shared_sums_over_molecule_boundaries(waters, count):
+    """Classes of over 2368 chunks and 96 a molecule: a CTA takes runs of chunks, some across two molecules.
+
+    The runs are 2 to 4 chunks and the molecules' counts no multiples of them
+    (114 (ss|s) chunks a (H2O)4, 249 (ss|p)); each molecule has its own
+    geometry and weights, so sums added to the neighbour show.
+    """
+    mols = [make_molecule(geometry.water_cluster(waters, np.random.default_rng([3, i])), "def2-svp",
+                          "cc-pvdz-jkfit") for i in range(count)]
+    _check_batch(mols, range(0, count, 4))
+
+
+def _weighted(plan, xyz, dens, wdens, mbar, abar, weight):
+    """The three energies whose derivatives the contractions are."""
+    f64 = dict(dtype=torch.float64, device="cuda")
+    s, t, v = (torch.empty(plan.mat_total, **f64) for _ in range(3))
+    m, a = (torch.empty(k, **f64) for k in (plan.met_total, plan.a_total))
+    _lib.call("vqc_int1e", plan.handle, xyz.data_ptr(), s.data_ptr(), t.data_ptr(), v.data_ptr(), _stream())
+    _lib.call("vqc_int2c", plan.handle, xyz.data_ptr(), m.data_ptr(), _stream())
+    _lib.call("vqc_int3c", plan.handle, xyz.data_ptr(), a.data_ptr(), _stream())
+    return torch.stack([(dens * (t + v)).sum() - (wdens * s).sum(), (mbar * m).sum(), (weight * abar * a).sum()])
+
+
+@pytest.mark.parametrize("pairs", [2, 64, 66])  # 4, 128 and 132 atoms: either side of the shared sums' limit
+def test_derivatives_against_differences(pairs):
+    rng = np.random.default_rng(pairs)
+    atoms = [("H", tuple(np.array([3.0 * (i // 2), 0.0, 0.75 * (i % 2)]) + 0.1 * rng.standard_normal(3)))
+             for i in range(2 * pairs)]
+    plan = NativePlan([make_molecule(atoms, "sto-3g", "cc-pvdz-jkfit")], True)
+    lay = plan.layout[0]
+    dens, wdens, mbar, abar = _weights(plan, pairs)
+    sym = lambda w, k: (w.view(k, k) + w.view(k, k).T).reshape(-1).contiguous()  # noqa: E731
+    dens, wdens, mbar = sym(dens, lay.nao), sym(wdens, lay.nao), sym(mbar, lay.naux)
+    off = torch.tril_indices(lay.nao, lay.nao, device="cuda")
+    weight = torch.where(off[0] == off[1], 1.0, 2.0).double().repeat_interleave(lay.naux)
+    grads = _gradients(plan, dens, wdens, mbar, abar)
+    x0 = torch.as_tensor(plan.coordinates(), device="cuda").contiguous()
+    h = 4e-3
+    for atom in (0, pairs, 2 * pairs - 1):
+        direction = torch.zeros_like(x0)
+        direction[atom] = torch.tensor([0.6, -0.48, 0.64], dtype=torch.float64)
+        f = {k: _weighted(plan, (x0 + k * h * direction).contiguous(), dens, wdens, mbar, abar, weight)
+             for k in (-2, -1, 1, 2)}
+        want = (8 * (f[1] - f[-1]) - (f[2] - f[-2])) / (12 * h)
+        for g, w in zip(grads, want):
+            # h^4 f'''''/30 with f''''' of the order of (2 a)^2 = 50 f': 5e-10;
+            # roundings of sums of up to 3e7 terms over h: below 1e-7
+            assert abs(float((g * direction).sum() - w)) < 1e-6 * (1.0 + float(g.abs().max()))
+    plan.close()
+
+
+def _cluster_plan():
+    return NativePlan([make_molecule(geometry.water_cluster(3, np.random.default_rng([4, i])), "def2-svp",
+                                     "cc-pvdz-jkfit") for i in range(2)], True)
+
+
+def test_classes_in_order_under_capture():
+    """Captured, the classes run in order on one stream: the same results as side by side."""
+    plan = _cluster_plan()
+    weights = _weights(plan, 5)
+    want, want_g = _integrals(plan), _gradients(plan, *weights)
+    xyz = torch.as_tensor(plan.coordinates(), device="cuda").contiguous()
+    out = [torch.zeros_like(w) for w in want]
+    grads = [torch.zeros_like(g) for g in want_g]
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        h, x, st = plan.handle, xyz.data_ptr(), _stream()
+        s, t, v, m, a = (o.data_ptr() for o in out)
+        _lib.call("vqc_int1e", h, x, s, t, v, st)
+        _lib.call("vqc_int2c", h, x, m, st)
+        _lib.call("vqc_int3c", h, x, a, st)
+        for g in grads:
+            g.zero_()
+        dens, wdens, mbar, abar = (w.data_ptr() for w in weights)
+        _lib.call("vqc_grad1e", h, x, dens, wdens, grads[0].data_ptr(), st)
+        _lib.call("vqc_grad2c", h, x, mbar, grads[1].data_ptr(), st)
+        _lib.call("vqc_grad3c", h, x, abar, grads[2].data_ptr(), st)
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, w) for o, w in zip(out, want))
+    for g, w in zip(grads, want_g):
+        assert (g - w).abs().max().item() <= 1e-12 * (1.0 + w.abs().max().item())
+    plan.close()
+
+
+def test_order_with_the_callers_stream():
+    """Inputs written late on the caller's stream, outputs read on it at once."""
+    plan = _cluster_plan()
+    want = _integrals(plan)
+    host = torch.as_tensor(plan.coordinates(), device="cuda").contiguous()
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        xyz = torch.zeros_like(host)
+        a = torch.zeros(plan.a_total, dtype=torch.float64, device="cuda")
+        torch.cuda._sleep(20_000_000)  # about 10 ms
+        xyz.copy_(host)
+        _lib.call("vqc_int3c", plan.handle, xyz.data_ptr(), a.data_ptr(), stream.cuda_stream)
+        got = a.clone()
+        xyz.zero_()  # the next work of the stream must not reach the kernels
+        a.zero_()
+    stream.synchronize()
+    assert torch.equal(got, want[4])
+    plan.close()
+
+
+def test_one_plan_in_two_threads():
+    """A call that finds the plan's streams taken runs in order on its own stream."""
+    plan = _cluster_plan()
+    want = _integrals(plan)
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work():
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(50):
+                got = _integrals(plan)
+                if not all(torch.equal(g, w) for g, w in zip(got, want)):
+                    wrong.append(1)
+        torch.cuda.synchronize()
+
+    threads = [threading.Thread(target=work) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    plan.close()

@@ -35,14 +35,28 @@ __device__ __forceinline__ void cart_of_g(int l, int k, int& x, int& y, int& z) 
 // Gradient sums of one molecule in shared memory.  A 3-centre CTA works
 // through a run of launch chunks and adds to global memory when the molecule
 // changes: one global atomic per atom, direction and run of chunks instead of
-// a few per warp.  Every CTA of a launch is on the same few molecules at a
-// time, so those atomics met on a handful of L2 sectors (12 x (H2O)6: (ss|s)
-// 0.226 -> 0.152 ms, (ps|s) 0.302 -> 0.211, (ps|p) 0.409 -> 0.299).  Molecules
-// of more atoms take the global atomics directly.
+// a few per warp.  Where every CTA of a launch is on the same few molecules at
+// a time, those atomics meet on a handful of L2 sectors (12 x (H2O)6: (ss|s)
+// 0.237 -> 0.144 ms, (ps|p) 0.418 -> 0.267).  Molecules of more atoms take the
+// global atomics directly.
 constexpr int kAccAtoms = 128;
+template <bool SHARED>
 struct AtomSums {
-  double v[3 * kAccAtoms];
+  double v[SHARED ? 3 * kAccAtoms : 1];
 };
+
+// The sums cost a CTA their zeroing, two barriers and a slower start, so they
+// are for the classes of short chunks, whose atomics come fast, and for
+// molecules of enough chunks to crowd them.  Other classes lose: (H2O)16
+// (pp|d) 0.377 -> 0.424 ms, (dd|p) 0.063 -> 0.071.
+__host__ __device__ constexpr bool shared_sums(int la, int lb, int lc) {
+  return la + lb + lc <= 2 || (lb == 0 && la <= 2 && lc <= 2 && la + lc <= 3);
+}
+// Chunks per molecule from which they pay, direct and shared: (ss|s) of
+// 185 x (H2O)3 (49 chunks each) 0.294 and 0.299 ms, of 78 x (H2O)4 (114) 0.336
+// and 0.289; (pp|s) of 40 x (H2O)5 (74) 0.143 and 0.145, of 9 x (H2O)8 (297)
+// 0.144 and 0.120; (ss|s) of 2048 single waters (2) 0.204 and 0.253.
+constexpr long long kSumChunks = 96;
 
 // Chunks a CTA works through: up to four, as long as eight CTAs per SM remain.
 // One chunk 3.79, two 3.71, four 3.63, eight 3.69, sixteen 3.63 ms for the
@@ -52,7 +66,7 @@ inline int chunks_per_cta(int nblocks) {
   return per < 1 ? 1 : (per < 4 ? per : 4);
 }
 
-__device__ __forceinline__ void flush_sums(AtomSums& acc, const DevMol& mol, double* __restrict__ grad) {
+__device__ __forceinline__ void flush_sums(AtomSums<true>& acc, const DevMol& mol, double* __restrict__ grad) {
   __syncthreads();
   for (int i = threadIdx.x; i < 3 * min(mol.natom, kAccAtoms); i += blockDim.x) {
     const double v = acc.v[i];
@@ -156,8 +170,8 @@ __global__ void __launch_bounds__(round32(Int3cCfg<LA, LB, LC, SPH>::THREADS),
                                   min_ctas_grad3c(LA, LB, LC))
     grad3c_kernel(DevBasis orb, DevBasis aux, const double* __restrict__ xyz,
                   const DevMol* __restrict__ mols, const int2* __restrict__ pairs,
-                  const ClassMol* __restrict__ cms, int ncm, int nblocks, int per_cta, int stride, const double* __restrict__ abar,
-                  double* __restrict__ grad) {
+                  const ClassMol* __restrict__ cms, int ncm, int nblocks, int per_cta,
+                  bool use_sums, int stride, const double* __restrict__ abar, double* __restrict__ grad) {
   using C = Int3cCfg<LA, LB, LC, SPH>;
   constexpr int NCA = ncart(LA), NCB = ncart(LB), NCC = ncart(LC);
   constexpr int NOA = C::NOA, NOB = C::NOB, NOC = C::NOC;
@@ -167,21 +181,25 @@ __global__ void __launch_bounds__(round32(Int3cCfg<LA, LB, LC, SPH>::THREADS),
   constexpr Cart<LB> cb{};
 
   __shared__ __align__(16) PairTable tab;
-  __shared__ AtomSums sums;
-  for (int i = threadIdx.x; i < 3 * kAccAtoms; i += blockDim.x) sums.v[i] = 0.0;
+  constexpr bool SHARED = shared_sums(LA, LB, LC);
+  __shared__ AtomSums<SHARED> sums;
+  if (SHARED && use_sums)
+    for (int i = threadIdx.x; i < 3 * kAccAtoms; i += blockDim.x) sums.v[i] = 0.0;
   int held = -1, first = 0;  // molecule the sums belong to, its first atom
   bool local = false;
   auto add = [&](int i, double v) {
-    if (local) atomicAdd(&sums.v[i - 3 * first], v);
+    if (SHARED && local) atomicAdd(&sums.v[i - 3 * first], v);
     else atomicAdd(grad + i, v);
   };
   for (int block = blockIdx.x * per_cta; block < min(nblocks, ((int)blockIdx.x + 1) * per_cta); ++block) {
     const ClassMol cm = cms[find_cm(cms, ncm, block)];
-    if (cm.mol != held) {
-      if (local) flush_sums(sums, mols[held], grad);
-      held = cm.mol;
-      first = mols[held].atom_off;
-      local = mols[held].natom <= kAccAtoms;
+    if constexpr (SHARED) {
+      if (use_sums && cm.mol != held) {
+        if (local) flush_sums(sums, mols[held], grad);
+        held = cm.mol;
+        first = mols[held].atom_off;
+        local = mols[held].natom <= kAccAtoms;
+      }
     }
     const int t0 = (block - cm.chunk_begin) * C::SLOTS;
     const int slot = threadIdx.x / NCC, kc = threadIdx.x % NCC;
@@ -266,7 +284,9 @@ __global__ void __launch_bounds__(round32(Int3cCfg<LA, LB, LC, SPH>::THREADS),
     warp_seg_add(add, atomB, gB[0], gB[1], gB[2]);
     warp_seg_add(add, atomC, -(gA[0] + gB[0]), -(gA[1] + gB[1]), -(gA[2] + gB[2]));
   }
-  if (local) flush_sums(sums, mols[held], grad);
+  if constexpr (SHARED) {
+    if (local) flush_sums(sums, mols[held], grad);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -293,8 +313,8 @@ __global__ void __launch_bounds__(rp_threads_g3c(LA, LB, LC, SPH),
                                   min_ctas_rp(rp_threads_g3c(LA, LB, LC, SPH), LA + LB + LC))
     grad3c_rp_kernel(DevBasis orb, DevBasis aux, const double* __restrict__ xyz,
                      const DevMol* __restrict__ mols, const int2* __restrict__ pairs,
-                     const ClassMol* __restrict__ cms, int ncm, int nblocks, int per_cta, int stride, const double* __restrict__ abar,
-                     double* __restrict__ grad) {
+                     const ClassMol* __restrict__ cms, int ncm, int nblocks, int per_cta,
+                     bool use_sums, int stride, const double* __restrict__ abar, double* __restrict__ grad) {
   using C = Int3cCfg<LA, LB, LC, SPH>;
   constexpr int NCA = ncart(LA), NCB = ncart(LB), NCC = ncart(LC);
   constexpr int NOA = C::NOA, NOB = C::NOB, NOC = C::NOC;
@@ -306,21 +326,25 @@ __global__ void __launch_bounds__(rp_threads_g3c(LA, LB, LC, SPH),
   constexpr Cart<LC> cc{};
 
   __shared__ __align__(16) PairTable tab;
-  __shared__ AtomSums sums;
-  for (int i = threadIdx.x; i < 3 * kAccAtoms; i += blockDim.x) sums.v[i] = 0.0;
+  constexpr bool SHARED = shared_sums(LA, LB, LC);
+  __shared__ AtomSums<SHARED> sums;
+  if (SHARED && use_sums)
+    for (int i = threadIdx.x; i < 3 * kAccAtoms; i += blockDim.x) sums.v[i] = 0.0;
   int held = -1, first = 0;  // molecule the sums belong to, its first atom
   bool local = false;
   auto add = [&](int i, double v) {
-    if (local) atomicAdd(&sums.v[i - 3 * first], v);
+    if (SHARED && local) atomicAdd(&sums.v[i - 3 * first], v);
     else atomicAdd(grad + i, v);
   };
   for (int block = blockIdx.x * per_cta; block < min(nblocks, ((int)blockIdx.x + 1) * per_cta); ++block) {
     const ClassMol cm = cms[find_cm(cms, ncm, block)];
-    if (cm.mol != held) {
-      if (local) flush_sums(sums, mols[held], grad);
-      held = cm.mol;
-      first = mols[held].atom_off;
-      local = mols[held].natom <= kAccAtoms;
+    if constexpr (SHARED) {
+      if (use_sums && cm.mol != held) {
+        if (local) flush_sums(sums, mols[held], grad);
+        held = cm.mol;
+        first = mols[held].atom_off;
+        local = mols[held].natom <= kAccAtoms;
+      }
     }
     const int t0 = (block - cm.chunk_begin) * C::SLOTS;
     const int slot = threadIdx.x / NR, r = threadIdx.x % NR;
@@ -428,7 +452,9 @@ __global__ void __launch_bounds__(rp_threads_g3c(LA, LB, LC, SPH),
     warp_seg_add(add, atomB, gB[0], gB[1], gB[2]);
     warp_seg_add(add, atomC, -(gA[0] + gB[0]), -(gA[1] + gB[1]), -(gA[2] + gB[2]));
   }
-  if (local) flush_sums(sums, mols[held], grad);
+  if constexpr (SHARED) {
+    if (local) flush_sums(sums, mols[held], grad);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -538,7 +564,7 @@ __global__ void __launch_bounds__(128)
   constexpr int MODE = SPH ? 0 : 1;
   constexpr Cart<LA> ca{};
   constexpr Cart<LB> cb{};
-  __shared__ AtomSums sums;
+  __shared__ AtomSums<true> sums;
   for (int i = threadIdx.x; i < 3 * kAccAtoms; i += blockDim.x) sums.v[i] = 0.0;
   __syncthreads();
   const ClassMol cm = cms[find_cm(cms, ncm, blockIdx.x)];
@@ -715,13 +741,14 @@ __global__ void __launch_bounds__(128)
 
 template <int LA, int LB, int LC, bool SPH>
 static void glaunch3(const ClassLaunch& cl, const KernelArgs& k, cudaStream_t st) {
-  const int per = chunks_per_cta(cl.nblocks), grid = (cl.nblocks + per - 1) / per;
+  const bool sums = shared_sums(LA, LB, LC) && cl.nblocks >= kSumChunks * cl.ncm;
+  const int per = sums ? chunks_per_cta(cl.nblocks) : 1, grid = (cl.nblocks + per - 1) / per;
   if constexpr (use_root_parallel_g3c(LA, LB, LC)) {
     grad3c_rp_kernel<LA, LB, LC, SPH><<<grid, rp_threads_g3c(LA, LB, LC, SPH), 0, st>>>(
-        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, cl.nblocks, per, cl.nab, k.w1, k.grad);
+        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, cl.nblocks, per, sums, cl.nab, k.w1, k.grad);
   } else {
     grad3c_kernel<LA, LB, LC, SPH><<<grid, round32(Int3cCfg<LA, LB, LC, SPH>::THREADS), 0, st>>>(
-        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, cl.nblocks, per, cl.nab, k.w1, k.grad);
+        k.orb, k.aux, k.xyz, k.mols, cl.pairs, cl.cms, cl.ncm, cl.nblocks, per, sums, cl.nab, k.w1, k.grad);
   }
 }
 
