@@ -231,9 +231,12 @@ int vqc_sp2_update(const double* x, const double* x2, double* xout, int32_t nmol
  * Whole SP2 purification of nmol symmetric n*n blocks fo (row-major,
  * contiguous; the mean of fo and its transpose is used) in one launch:
  * Gershgorin map to [0, 1], then X^2 or 2X - X^2 steps as above until
- * |tr X - tr X^2| < tol or max_steps steps; out receives X, the projector onto
- * the lowest nocc eigenvectors.  path: 0 picks by size; 1 one CTA per molecule
- * (n <= 112); 2, 3 cooperative groups of CTAs with 32- and 64-row tiles.
+ * |tr X - tr X^2| < tol, and then one X^2 and one 2X - X^2 step more, or until
+ * max_steps steps; out receives X, the projector onto the lowest nocc
+ * eigenvectors: zero for nocc <= 0, the identity for nocc >= n, and NaN for a
+ * multiple of the identity with a nocc between, which has no such projector.
+ * path: 0 picks by size; 1 one CTA per molecule (n <= 112); 2, 3 cooperative
+ * groups of CTAs with 32- and 64-row tiles.
  * Groups need a workspace of vqc_sp2_purify_workspace bytes (256-byte
  * aligned, contents undefined); error receives 31 if a group's barrier
  * expires (it is not written otherwise; the caller zeroes it).

@@ -95,3 +95,32 @@ def test_one_large_molecule_uses_every_cta(n):
             best = min(best, a.elapsed_time(b))
         times.append(best)
     assert times[0] < times[1], times
+
+
+@pytest.mark.parametrize("path", [0, 1, 2, 3])
+def test_bounds_that_are_eigenvalues(path):
+    """One function, multiples of the identity and diagonal matrices: the map has no room beside the spectrum."""
+    f64 = dict(dtype=torch.float64, device="cuda")
+    for n in (1, 5, 70):
+        eye = torch.eye(n, **f64).expand(3, n, n)
+        for f in (-0.9 * eye, torch.zeros(3, n, n, **f64), torch.diag(torch.linspace(-2.0, 1.0, n, **f64)).expand(3, n, n)):
+            f = f.contiguous()
+            assert torch.equal(_purify_fp64(f, n, 96, 1e-11, path), eye)
+            assert torch.equal(_purify_fp64(f, 0, 96, 1e-11, path), torch.zeros_like(f))
+        bad = f.clone()
+        bad[1, 0, n - 1] = float("nan")
+        got = _purify_fp64(bad, n, 96, 1e-11, path)
+        assert torch.isnan(got[1, 0, n - 1]) and torch.equal(got[0], eye[0]) and torch.equal(got[2], eye[2])
+    # one of two degenerate levels: no projector, and none is made up
+    assert torch.isnan(_purify_fp64(torch.eye(2, **f64)[None].contiguous(), 1, 96, 1e-11, path)).any()
+    f = torch.diag(torch.tensor([-2.0, -1.0, 0.5, 1.0], **f64))[None].contiguous()
+    want = torch.diag(torch.tensor([1.0, 1.0, 0.0, 0.0], **f64))[None]
+    assert (_purify_fp64(f, 2, 96, 1e-11, path) - want).abs().max().item() < 1e-12
+
+
+@pytest.mark.parametrize("gemm", ["fp64", "int8"])
+def test_everything_occupied_in_either_form(gemm):
+    f = torch.diag(torch.tensor([-2.0, -1.0, -1.0], dtype=torch.float64, device="cuda"))[None].contiguous()
+    eye = torch.eye(3, dtype=torch.float64, device="cuda")[None]
+    assert torch.equal(purify_sp2(f, 3, gemm=gemm), eye)
+    assert torch.equal(purify_sp2(f, 0, gemm=gemm), torch.zeros_like(f))

@@ -440,6 +440,21 @@ __global__ void __launch_bounds__(GroupCfg<BM>::THREADS, GroupCfg<BM>::CTAS)
   }
 }
 
+// Nothing or everything occupied: zero or the identity, whatever the spectrum.
+// The steps cannot reach the identity where a Gershgorin bound is an
+// eigenvalue (it is mapped to 0 and stays there), as for one function or a
+// diagonal matrix.  Non-finite elements stay visible.
+__global__ void __launch_bounds__(256)
+    sp2_trivial_kernel(const double* __restrict__ fo, size_t total, int n, double diagonal,
+                       double* __restrict__ out) {
+  for (size_t e = (size_t)blockIdx.x * 256 + threadIdx.x; e < total; e += (size_t)gridDim.x * 256) {
+    const size_t nn = (size_t)n * n, base = e / nn * nn;
+    const int i = (int)((e - base) / n), j = (int)((e - base) % n);
+    const double sum = fo[e] + fo[base + (size_t)j * n + i];
+    out[e] = (i == j ? diagonal : 0.0) + 0.0 * sum;
+  }
+}
+
 struct Choice {
   int path;  // 1: one CTA per molecule; 2, 3: groups with 32- and 64-row tiles
   int ngroups, G;
@@ -538,6 +553,13 @@ int vqc_sp2_purify(const double* fo, int32_t nmol, int32_t n, double nocc, doubl
       (path == 1 && n > sp2::kSmallMaxN))
     return fail(VQC_STATUS_INVALID_ARGUMENT, "sp2_purify: bad argument");
   cudaStream_t st = (cudaStream_t)stream;
+  if (nocc <= 0.0 || nocc >= n) {
+    const size_t total = (size_t)nmol * n * n, ctas = (total + 255) / 256;
+    sp2::sp2_trivial_kernel<<<(int)(ctas > 16 * 148 ? 16 * 148 : ctas), 256, 0, st>>>(
+        fo, total, n, nocc <= 0.0 ? 0.0 : 1.0, out);
+    count_launch();
+    return cuda_status(cudaGetLastError(), "sp2_purify");
+  }
   sp2::Choice ch{};
   cudaError_t e = sp2::choose(nmol, n, path, ch);
   if (e != cudaSuccess) return cuda_status(e, "sp2_purify");

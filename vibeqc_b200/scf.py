@@ -300,8 +300,9 @@ def purify_sp2(fo: torch.Tensor, nocc: int, max_steps: int = 96, tol: float = 1e
     Second-order spectral projection (Niklasson, Phys. Rev. B 66, 155115
     (2002)): map the spectrum into [0, 1] with Gershgorin bounds, then apply
     X <- X^2 or X <- 2X - X^2, whichever moves tr X toward ``nocc``, until
-    tr(X) - tr(X^2) < tol.  With ``gemm="fp64"`` the whole purification is one
-    native launch (vqc_sp2_purify).  ``gemm="int8"`` forms X^2 from sliced
+    tr(X) - tr(X^2) < tol.  With ``gemm="fp64"``, or nothing or everything
+    occupied, the whole purification is one native launch (vqc_sp2_purify),
+    which ends with two steps more.  ``gemm="int8"`` forms X^2 from sliced
     tensor-core products, in CUDA graphs of ``steps`` (even) steps cached in
     ``graphs``, one per shape and tolerance; the convergence flags stay on the
     device and are read once per graph replay.
@@ -309,7 +310,7 @@ def purify_sp2(fo: torch.Tensor, nocc: int, max_steps: int = 96, tol: float = 1e
     nb, n, _ = fo.shape
     # the cap counts whole groups of ``steps``, as the graphs run them
     cap = -(-max_steps // int(steps)) * int(steps)
-    if gemm != "int8":
+    if gemm != "int8" or not 0 < nocc < n:
         return _purify_fp64(fo, nocc, cap, tol)
     diag = torch.diagonal(fo, dim1=1, dim2=2)
     radius = fo.abs().sum(dim=2) - diag.abs()
