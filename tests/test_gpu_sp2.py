@@ -1,9 +1,9 @@
-"""Purification with the X^2 product on the int8 tensor cores against the DGEMM form.
+"""Purification with the X^2 product on the int8 tensor cores against the FP64 form.
 
 SP2 (Niklasson, PRB 66, 155115 (2002)) needs X^2 to FP64 accuracy in the
 anchored phase of the mixed SCF (density tolerance 1e-8); the sliced int8
 product (7-bit slices, exact int32 accumulation) must give the same
-projector as the batched DGEMM, and a mixed-precision SCF that purifies with
+projector as the FP64 products, and a mixed-precision SCF that purifies with
 it must reproduce the FP64 path's energies and forces.
 """
 

@@ -5,6 +5,8 @@ K stages and of the one-CTA form; batches at one molecule, several groups and
 more molecules than resident groups.
 """
 
+import threading
+
 import pytest
 import torch
 
@@ -124,3 +126,25 @@ def test_everything_occupied_in_either_form(gemm):
     eye = torch.eye(3, dtype=torch.float64, device="cuda")[None]
     assert torch.equal(purify_sp2(f, 3, gemm=gemm), eye)
     assert torch.equal(purify_sp2(f, 0, gemm=gemm), torch.zeros_like(f))
+
+
+@pytest.mark.parametrize("nb,n", [(4, 264), (1, 512), (40, 64)])
+def test_two_threads_at_once(nb, n):
+    """Each launch brings its own workspace, and a cooperative launch is resident as a whole."""
+    f, _ = _fock(nb, n, n // 5, n)
+    want = _purify_fp64(f, n // 5, 96, 1e-11)
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work():
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(10):
+                if not torch.equal(_purify_fp64(f, n // 5, 96, 1e-11), want):
+                    wrong.append(1)
+
+    threads = [threading.Thread(target=work) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong

@@ -13,8 +13,8 @@ series of degree DEG on intervals of width H (nodes at Chebyshev points),
 expands the series in powers of x in [-1, 1] (still in 80 digits; the series
 falls so fast that the powers lose nothing) and writes the coefficients as hex
 doubles into ``rys_table.inc``: per interval and root, from the highest power
-down, (u, w) coefficient pairs, so that a Horner step of both takes one 16-byte
-load.  For
+down, (u, w) coefficient pairs, so that one 32-byte load brings two Horner steps
+of both.  For
 T >= T_asym(n) the kernels use the large-T limit u_i = x_i^2 / T,
 w_i = W_i / sqrt(T) with (x_i, W_i) the positive Gauss-Hermite nodes/weights of
 order 2n; those constants are written too.  T_asym(n) is the smallest grid

@@ -2,14 +2,18 @@
 //
 // sp2_update: one step of second-order spectral projection (Niklasson,
 // Phys. Rev. B 66, 155115 (2002)) for every molecule of a chunk, given
-// X and X2 = X X (a batched GEMM).  Each CTA recomputes tr X and tr X^2 of its
-// molecule, chooses X^2 or 2X - X^2 (whichever moves tr X toward n_occ) and
-// writes its slice of the next iterate to a separate buffer.  A molecule whose
-// idempotency error |tr X - tr X^2| fell below tol is copied unchanged and
-// flagged, so a fixed number of steps can run without host synchronisation.  Replaces the per-iteration
-// batched eigensolver of the reference's device SCF loop
-// (src/scf/cuda/df_scf_library.cpp, cusolverDnXsyevBatched) for the density
-// update.
+// X and X2 = X X.  It serves the purification whose X X is a sliced int8
+// product (ozaki_gemm.cu); the FP64 purification, which updates the density by
+// default, is one launch of its own (sp2_purify.cu).  Each CTA recomputes tr X
+// and tr X^2 of its molecule, chooses X^2 or 2X - X^2 (whichever moves tr X
+// toward n_occ) and writes its slice of the next iterate to a separate buffer.
+// A molecule whose idempotency error |tr X - tr X^2| fell below tol is copied
+// unchanged and flagged, so a fixed number of steps can run without host
+// synchronisation.  Purification replaces the per-iteration batched eigensolver
+// of the reference's device SCF loop (src/scf/cuda/df_scf_library.cpp,
+// cusolverDnXsyevBatched).
+//
+// scf_change, scf_record: convergence test and bookkeeping of an iteration.
 #include "vqc_df.h"
 #include "vqc_kernels.cuh"
 #include "vqc_plan.hpp"

@@ -791,8 +791,8 @@ def run_scf(chunk: Chunk, ints: ChunkIntegrals, xyz: torch.Tensor, *, precision:
     guess = torch.randn(nb, n, nocc, dtype=torch.float64, device=dev, generator=gen)
 
     sp2_graphs = _SP2_GRAPHS
-    # the FP64 comparator path keeps plain DGEMMs; the mixed path may take
-    # the sliced tensor-core products (FP64-accurate as well)
+    # the FP64 path purifies in one FP64 launch; the mixed path may take the
+    # sliced tensor-core products instead (FP64-accurate as well)
     sp2_gemm = sched.sp2_gemm if precision == "mixed" else "fp64"
 
     def density_from(f, guess, tol=1e-11, noise_scale=0.3):
