@@ -280,3 +280,21 @@ def test_one_plan_in_two_threads():
         t.join()
     assert not wrong
     plan.close()
+
+
+def test_full_batches_of_heavy_atoms():
+    """512 against 32 molecules of six argon atoms: below six times the time.
+
+    32 leave the GPU half empty; with eight lanes a pair, most without work of
+    their own, 512 took eight times as long, with two lanes they take four.
+    """
+    mol = make_molecule([("Ar", (7.0 * (i % 3), 7.0 * (i // 3), 0.2 * i)) for i in range(6)], "sto-3g", "def2-tzvp")
+    times = []
+    for count in (32, 512):
+        plan = NativePlan([mol] * count, True)
+        xyz = torch.as_tensor(plan.coordinates(), device="cuda").contiguous()
+        out = [torch.empty(plan.mat_total, dtype=torch.float64, device="cuda") for _ in range(3)]
+        times.append(_time(lambda: _lib.call("vqc_int1e", plan.handle, xyz.data_ptr(),
+                                             *(o.data_ptr() for o in out), _stream())))
+        plan.close()
+    assert times[1] < 6 * times[0], times

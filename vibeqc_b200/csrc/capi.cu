@@ -224,7 +224,7 @@ int Plan::build(const vqc_batch_desc& d) {
     ClassMol* dcm = nullptr;
     int s2 = upload(owned, cms, &dcm);
     if (s2) return s2;
-    list.push_back(ClassLaunch{la, lb, lc, nab, pairs, dcm, (int)cms.size(), nb});
+    list.push_back(ClassLaunch{la, lb, lc, nab, lanes_1e(nb, natom / nmol), pairs, dcm, (int)cms.size(), nb});
     return VQC_STATUS_SUCCESS;
   };
   for (int la = 0; la <= kMaxKernelL; ++la)

@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(128)
     if (local) atomicAdd(&sums.v[i - 3 * mol.atom_off], v);
     else atomicAdd(grad + i, v);
   };
-  const Lanes1e ln(mol.natom);
+  const Lanes1e<k1eLanes> ln(mol.natom);
   const int2 pr = pairs[cm.pair_begin + (valid ? t : 0)];
   const int atomA = orb.atom[pr.x], atomB = orb.atom[pr.y];
   const double factor = (pr.x == pr.y) ? 1.0 : 2.0;

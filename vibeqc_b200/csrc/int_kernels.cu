@@ -421,21 +421,21 @@ __device__ __forceinline__ void store_1e(int mode, const double (&acc)[ncart(LA)
     }
 }
 
-// sum over the lanes of a pair (k1eLanes consecutive lanes), in every lane
-template <int NCA, int NCB>
+// sum over the lanes of a pair (LANES consecutive lanes), in every lane
+template <int LANES, int NCA, int NCB>
 __device__ __forceinline__ void lanes_sum(double (&acc)[NCA][NCB]) {
 #pragma unroll
   for (int i = 0; i < NCA; ++i)
 #pragma unroll
     for (int j = 0; j < NCB; ++j)
 #pragma unroll
-      for (int off = 1; off < k1eLanes; off <<= 1) acc[i][j] += __shfl_xor_sync(0xffffffffu, acc[i][j], off);
+      for (int off = 1; off < LANES; off <<= 1) acc[i][j] += __shfl_xor_sync(0xffffffffu, acc[i][j], off);
 }
 
-// k1eLanes lanes per shell pair: they share its primitive pairs for S and T,
+// LANES lanes per shell pair: they share its primitive pairs for S and T,
 // and its (primitive pair, nucleus) products for V (Lanes1e)
-template <int LA, int LB, bool SPH>
-__global__ void __launch_bounds__(128)
+template <int LA, int LB, bool SPH, int LANES>
+__global__ void __launch_bounds__(k1ePairs * LANES)
     int1e_kernel(DevBasis orb, const double* __restrict__ xyz, const double* __restrict__ charge,
                  const DevMol* __restrict__ mols, const int2* __restrict__ pairs,
                  const ClassMol* __restrict__ cms, int ncm, double* __restrict__ S,
@@ -447,10 +447,10 @@ __global__ void __launch_bounds__(128)
   constexpr Cart<LA> ca{};
   constexpr Cart<LB> cb{};
   const ClassMol cm = cms[find_cm(cms, ncm, blockIdx.x)];
-  const int t = (blockIdx.x - cm.chunk_begin) * k1ePairs + threadIdx.x / k1eLanes;
+  const int t = (blockIdx.x - cm.chunk_begin) * k1ePairs + threadIdx.x / LANES;
   const bool valid = t < cm.ntriples;
   const DevMol mol = mols[cm.mol];
-  const Lanes1e ln(mol.natom);
+  const Lanes1e<LANES> ln(mol.natom);
   const int2 pr = pairs[cm.pair_begin + (valid ? t : 0)];
   const double* A = xyz + 3 * orb.atom[pr.x];
   const double* B = xyz + 3 * orb.atom[pr.y];
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(128)
   for (int i = 0; i < NCA; ++i)
 #pragma unroll
     for (int j = 0; j < NCB; ++j) accs[i][j] = acct[i][j] = 0.0;
-  for (int k = ln.lane; k < nab; k += k1eLanes) {
+  for (int k = ln.lane; k < nab; k += LANES) {
     const int ia = pa0 + k / nb, ib = pb0 + k % nb;
     const double a = orb.exps[ia], b = orb.exps[ib];
     const double p = a + b, ip = 1.0 / p;
@@ -514,8 +514,8 @@ __global__ void __launch_bounds__(128)
                          acct[i][j]);
       }
   }
-  lanes_sum(accs);
-  lanes_sum(acct);
+  lanes_sum<LANES>(accs);
+  lanes_sum<LANES>(acct);
   if (valid && ln.lane == 0) store_1e<LA, LB, NOA, NOB>(MODE, accs, orb, pr, mol, S);
   if (valid && ln.lane == 1) store_1e<LA, LB, NOA, NOB>(MODE, acct, orb, pr, mol, T);
 
@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(128)
       }
     }
   }
-  lanes_sum(accv);
+  lanes_sum<LANES>(accv);
   if (valid && ln.lane == 0) store_1e<LA, LB, NOA, NOB>(MODE, accv, orb, pr, mol, V);
 }
 
@@ -585,8 +585,11 @@ static void launch2(const ClassLaunch& cl, const KernelArgs& k, cudaStream_t st)
 
 template <int LA, int LB, bool SPH>
 static void launch1(const ClassLaunch& cl, const KernelArgs& k, cudaStream_t st) {
-  int1e_kernel<LA, LB, SPH><<<cl.nblocks, 128, 0, st>>>(k.orb, k.xyz, k.charge, k.mols, cl.pairs, cl.cms,
-                                                        cl.ncm, k.out, k.out2, k.out3);
+  auto* kernel = cl.lanes == k1eFewLanes ? int1e_kernel<LA, LB, SPH, k1eFewLanes>
+                                         : int1e_kernel<LA, LB, SPH, k1eLanes>;
+  const int threads = k1ePairs * (cl.lanes == k1eFewLanes ? k1eFewLanes : k1eLanes);
+  kernel<<<cl.nblocks, threads, 0, st>>>(k.orb, k.xyz, k.charge, k.mols, cl.pairs, cl.cms, cl.ncm, k.out, k.out2,
+                                         k.out3);
 }
 
 #define VQC_L3(LA, LB, LC)                                              \

@@ -18,7 +18,8 @@ struct ClassMol {
 
 struct ClassLaunch {
   int la, lb, lc;
-  int nab;  // largest primitive count of the class's orbital pairs
+  int nab;    // 3-centre: largest primitive count of the class's orbital pairs
+  int lanes;  // 1-electron values: lanes per shell pair
   const int2* pairs;
   const ClassMol* cms;
   int ncm;
@@ -210,12 +211,26 @@ __device__ __forceinline__ int find_cm(const ClassMol* __restrict__ cms, int ncm
 // waters 6.4 -> 2.2 ms, 32768 H2 0.58 -> 0.14 (one lane a pair 2.2 and 0.22).
 constexpr int k1eLanes = 8;
 constexpr int k1ePairs = 128 / k1eLanes;
+// Where the pairs alone fill the GPU, lanes beyond the nuclei only add loads,
+// shuffles and the transforms' idle ones: values then take two lanes a pair
+// (512 x Ar6 STO-3G 0.281 -> 0.143 ms, one lane 0.214; 2048 x Ar2 def2-SVP
+// 0.327 -> 0.235).  The chunks a class must have grow with the nuclei, whose
+// loop is the tail: eight and two lanes 0.082 / 0.088 for 32 x (H2O)4 (832 (ss)
+// chunks), 0.126 / 0.119 for 64 (1664), 0.339 / 0.325 for 32 x (H2O)9 (4032),
+// 0.318 / 0.382 for 8 x (H2O)16 (3168).  Derivatives stay ahead with eight.
+constexpr int k1eFewLanes = 2;
+inline int lanes_1e(int nblocks, int atoms_per_molecule) {
+  return nblocks >= 1024 && nblocks / 170 >= atoms_per_molecule ? k1eFewLanes : k1eLanes;
+}
+
+template <int LANES>
 struct Lanes1e {
   int lane, c0, dc, k0, dk;
   __device__ __forceinline__ explicit Lanes1e(int natom) {
-    lane = threadIdx.x % k1eLanes;
-    dc = natom <= 1 ? 1 : (natom <= 2 ? 2 : (natom <= 4 ? 4 : 8));
-    dk = k1eLanes / dc;
+    lane = threadIdx.x % LANES;
+    dc = 1;
+    while (dc < LANES && dc < natom) dc *= 2;
+    dk = LANES / dc;
     c0 = lane % dc;
     k0 = lane / dc;
   }
