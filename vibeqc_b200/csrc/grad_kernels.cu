@@ -60,7 +60,8 @@ constexpr long long kSumChunks = 96;
 
 // Chunks a CTA works through: up to four, as long as eight CTAs per SM remain.
 // One chunk 3.79, two 3.71, four 3.63, eight 3.69, sixteen 3.63 ms for the
-// derivatives of 12 x (H2O)6; 1 x (H2O)16 4.79, 4.58, 4.56, 4.51, 4.55.
+// derivatives of 12 x (H2O)6; 1 x (H2O)16 4.79, 4.58, 4.56, 4.51, 4.55 (every
+// class summing in shared memory; CTAs that do not take one chunk).
 inline int chunks_per_cta(int nblocks) {
   const int per = nblocks / (148 * 8);
   return per < 1 ? 1 : (per < 4 ? per : 4);

@@ -486,7 +486,7 @@ __device__ __forceinline__ void slice_digits(double y0, int (&dig)[kMaxSlices]) 
 // warp; one-byte stores and the rounding / clamping / conversion chain held
 // the earlier form to 1.5 TB/s).  The row maximum enters only through its
 // exponent, so the first pass is an integer maximum over exponent fields.
-// 8 x (H2O)10: 2.65 -> 1.39 ms, 2.9 TB/s; the 21 FP64 operations an element
+// 8 x (H2O)10: 2.65 -> 1.18 ms, 3.4 TB/s; the 21 FP64 operations an element
 // takes are next.
 // VEC: 16-byte aligned source and scale rows and 4-byte aligned slice rows.
 // NS: the slice count; a count known only at run time costs the digit loop its

@@ -1,7 +1,7 @@
 // Whole SP2 purification (Niklasson, Phys. Rev. B 66, 155115 (2002)) of a batch
 // of equally sized symmetric FP64 matrices in one launch: Gershgorin bounds,
 // the map of the spectrum into [0, 1], every X <- X^2 or 2X - X^2 step until
-// |tr X - tr X^2| < tol, and the projector out.
+// |tr X - tr X^2| < tol and kPolish steps more, and the projector out.
 //
 // X stays exactly symmetric, so a step forms only the tiles on or above the
 // diagonal (half the flops of a plain product) and mirrors them, and
@@ -11,7 +11,7 @@
 // pipe (mma.m8n8k4, the same FP64 FMA rate as the scalar pipe at a quarter of
 // its operand reads).
 //
-// Two forms, chosen by sp2_choose below:
+// Two forms, chosen by choose() below:
 //   sp2_small_kernel  one CTA per molecule, X double-buffered in shared memory;
 //     steps are separated by one __syncthreads.  Bound by one SM's FP64 rate
 //     and, for the smallest, by the step's latency chain.
@@ -22,9 +22,9 @@
 //
 // Measured on B200 against a batched DGEMM and an update kernel per step in
 // 8-step graphs with a host read of the flags after each: 14 x N = 312
-// 2.73 -> 1.73 ms a purification; the purifications of one water molecule's
-// SCF (N = 24, 14 of them) 2.55 -> 0.57 ms of GPU time and five host reads
-// fewer each.
+// 2.72 -> 1.72 ms a purification, 1 x N = 1000 4.7 -> 2.8; the purifications of
+// one water molecule's SCF (N = 24, 14 of them) 2.55 -> 0.61 ms of GPU time and
+// five host reads fewer each.
 #include "vqc_df.h"
 #include "vqc_kernels.cuh"
 #include "vqc_plan.hpp"
@@ -462,7 +462,11 @@ struct Choice {
 
 // Groups of G CTAs for nmol molecules in r rounds, minimising the step time
 // r * (barrier + tiles per CTA * tile time): a tile of BM rows costs BM^2 n
-// FMAs at one SM's 64 a cycle, shared by the CTAs resident on it.
+// FMAs at one SM's 64 a cycle, shared by the CTAs resident on it.  The cycles
+// of a barrier (4000) and of filling a tile's pipeline (1500) and the factor
+// on the FMAs (1.4) are round numbers that rank plans: of 32- and 64-row tiles
+// the pick was the faster, or within 1 %, at 51 of 52 pairs of N = 120-2000
+// and 1-128 molecules (32 x N = 312: 3.08 against 2.91 ms).
 static Choice plan_groups(int nmol, int n, int bm, int resident, int sms, double& cost) {
   const int nt = (n + bm - 1) / bm, tiles = nt * (nt + 1) / 2;
   Choice best{bm == 32 ? 2 : 3, 0, 0};
@@ -491,10 +495,10 @@ static cudaError_t choose(int nmol, int n, int path, Choice& ch) {
   cudaError_t e;
   if ((e = cudaGetDevice(&dev))) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev))) return e;
-  // Measured us a purification, one CTA against 32-row groups: N = 24 55 / 180,
-  // N = 64 112 / 231, N = 72 (128 molecules) 153 / 517, N = 96 267 / 277-299,
-  // 128 x N = 96 280 / 579; N = 112 351 / 302-340 for up to 8 molecules but
-  // 351 / 407 for 32 and 368 / 972 for 128, as one SM per molecule stays
+  // Measured us a purification, one CTA against 32-row groups: N = 24 57 / 176,
+  // N = 64 115 / 237, N = 72 (128 molecules) 158 / 542, N = 96 279 / 291-309,
+  // 128 x N = 96 294 / 599; N = 112 347-368 / 316-356 for up to 8 molecules but
+  // 366 / 427 for 32 and 383 / 1029 for 128, as one SM per molecule stays
   // cheaper once the molecules alone fill a good part of the GPU.
   if (path == 0 && (n <= 96 || (n <= kSmallMaxN && nmol >= 24))) path = 1;
   if (path == 1) {

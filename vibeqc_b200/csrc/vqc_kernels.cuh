@@ -207,14 +207,14 @@ __device__ __forceinline__ int find_cm(const ClassMol* __restrict__ cms, int ncm
 // lanes, the primitive pairs as well.  (ss) derivatives of 12 x (H2O)6 0.290 ->
 // 0.068 ms, (ps) 0.245 -> 0.082; (ss) values of 8 x (H2O)9 0.151 -> 0.056.
 // A CTA takes k1ePairs pairs of one molecule.  A CTA of 128 pairs spread over
-// eight launched ones left most of these empty for small molecules: 16384
-// waters 6.4 -> 2.2 ms, 32768 H2 0.58 -> 0.14 (one lane a pair 2.2 and 0.22).
+// eight launched ones left most of these empty for small molecules: values of
+// 16384 waters 6.4 -> 2.2 ms, derivatives 9.6 -> 3.7, of 32768 H2 0.58 -> 0.14
+// and 1.31 -> 0.40.
 constexpr int k1eLanes = 8;
 constexpr int k1ePairs = 128 / k1eLanes;
 // Where the pairs alone fill the GPU, lanes beyond the nuclei only add loads,
 // shuffles and the transforms' idle ones: values then take two lanes a pair
-// (512 x Ar6 STO-3G 0.281 -> 0.143 ms, one lane 0.214; 2048 x Ar2 def2-SVP
-// 0.327 -> 0.235).  The chunks a class must have grow with the nuclei, whose
+// (512 x Ar6 STO-3G 0.281 -> 0.143 ms, one lane 0.214; 16384 waters 2.2 -> 1.2).  The chunks a class must have grow with the nuclei, whose
 // loop is the tail: eight and two lanes 0.082 / 0.088 for 32 x (H2O)4 (832 (ss)
 // chunks), 0.126 / 0.119 for 64 (1664), 0.339 / 0.325 for 32 x (H2O)9 (4032),
 // 0.318 / 0.382 for 8 x (H2O)16 (3168).  Derivatives stay ahead with eight.
